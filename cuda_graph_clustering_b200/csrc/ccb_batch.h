@@ -35,9 +35,10 @@ enum BatchKind : int { kBatchRegisters = 0, kBatchStream = 1, kBatchIncremental 
 // Kernel instance of one descent bucket and its persistent grid.
 struct BatchShape {
   int kind = kBatchRegisters;
-  int k = 0;            // compile-time K of the register and streamed forms
+  bool window = false;  // the windowed descent in the place of the kind's own kernel
+  int k = 0;            // compile-time K of the register, streamed and windowed (k <= 8) forms
   int threads = 256;
-  int vpt = 4;          // register form
+  int vpt = 4;          // register forms; windowed: members per scan thread
   bool smem = false;    // register form: bitset in shared memory; streamed / incremental: state in shared memory
   size_t smem_bytes = 0;
   int blocks_per_sm = 0;  // tuned resident slots per SM (0: the occupancy limit)

@@ -8,6 +8,7 @@
 #include "ccb_descent_incremental.cuh"
 #include "ccb_descent_registers.cuh"
 #include "ccb_descent_stream.cuh"
+#include "ccb_descent_window.cuh"
 
 namespace ccb {
 namespace {
@@ -55,6 +56,17 @@ __global__ void __launch_bounds__(T, 1) kb_descent_stream(const BatchEntry* __re
   int entry, slot;
   while (ClaimItem(q, &s_item, entry, slot)) {
     DescentStream<K, T, S>(CurrentDescent(entries[entry]), slot);
+    __syncthreads();
+  }
+}
+
+template <int K, bool S>
+__global__ void __launch_bounds__(kWindowThreads, 1) kb_descent_window(const BatchEntry* __restrict__ entries,
+                                                                       BatchQueue q) {
+  __shared__ int s_item;
+  int entry, slot;
+  while (ClaimItem(q, &s_item, entry, slot)) {
+    DescentWindow<K, S, int16_t>(CurrentDescent(entries[entry]), slot);
     __syncthreads();
   }
 }
@@ -270,6 +282,14 @@ __global__ void __launch_bounds__(T, 1) kf_stream(const BatchEntry* __restrict__
   FlowLoop<T>(entries, flow, b, [](const DescentArgs<int16_t>& a, int slot) { DescentStream<K, T, S>(a, slot); });
 }
 
+template <int K, bool S>
+__global__ void __launch_bounds__(kWindowThreads, 1) kf_window(const BatchEntry* __restrict__ entries, FlowState* flow,
+                                                               FlowBucket b) {
+  FlowLoop<kWindowThreads>(entries, flow, b, [](const DescentArgs<int16_t>& a, int slot) {
+    DescentWindow<K, S, int16_t>(a, slot);
+  });
+}
+
 template <int T, bool S>
 __global__ void __launch_bounds__(T, 1024 / T) kf_incremental(const BatchEntry* __restrict__ entries, FlowState* flow,
                                                               FlowBucket b) {
@@ -322,6 +342,15 @@ template <bool kFlow, typename F>
 cudaError_t WithKernel(const BatchShape& s, F&& f) {
 #define CCB_PICK(KB, KF) \
   if constexpr (kFlow) { return f(KF); } else { return f(KB); }
+#define CCB_WINDOW(K)                                                                                   \
+  if (s.window && s.k == K) {                                                                           \
+    if (s.smem) { CCB_PICK((kb_descent_window<K, true>), (kf_window<K, true>)) }                        \
+    CCB_PICK((kb_descent_window<K, false>), (kf_window<K, false>))                                      \
+  }
+  CCB_WINDOW(2) CCB_WINDOW(3) CCB_WINDOW(4) CCB_WINDOW(5) CCB_WINDOW(6) CCB_WINDOW(7) CCB_WINDOW(8)
+  CCB_WINDOW(16) CCB_WINDOW(32) CCB_WINDOW(64)
+#undef CCB_WINDOW
+  if (s.window) return cudaErrorInvalidValue;
 #define CCB_REG(K, T, V)                                                                                \
   if (s.kind == kBatchRegisters && s.k == K && s.threads == T && s.vpt == V) {                         \
     if (s.smem) { CCB_PICK((kb_descent_registers<K, T, V, true>), (kf_registers<K, T, V, true>)) }     \

@@ -1,0 +1,59 @@
+// Instances and launcher of the windowed descent (ccb_descent_window.cuh).
+#include <cuda_runtime.h>
+
+#include "ccb_descent_window.cuh"
+#include "ccb_plans.h"
+
+namespace ccb {
+namespace {
+
+template <int K, bool S, typename GainT>
+cudaError_t Go(const SmallKPlan& p, const DescentArgs<GainT>& a, int grid, cudaStream_t st, bool configure) {
+  auto kernel = k_descent_window<K, S, GainT>;
+  if (configure) return RaiseDynamicSmem(kernel, p.smem_bytes);
+  if (grid > 0) kernel<<<grid, kWindowThreads, p.smem_bytes, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int kBound>
+cudaError_t ByPlacement(const SmallKPlan& p, const DescentArgs<int16_t>& a, int grid, cudaStream_t st, bool cfg) {
+  return p.smem_state ? Go<kBound, true>(p, a, grid, st, cfg) : Go<kBound, false>(p, a, grid, st, cfg);
+}
+
+}  // namespace
+
+bool PlanWindow(SmallKPlan& p, int n, int k, size_t limit) {
+  constexpr size_t kStatic = 12 * 1024;  // the kernels' static shared memory
+  if (limit < kStatic) return false;
+  limit -= kStatic;
+  p.window = true;
+  p.k = WindowBound(k);
+  p.threads = kWindowThreads;
+  p.registers = false;
+  p.smem_rows = false;
+  p.vpt = WindowFormOf(p.k).Members();
+  p.smem_state = WindowSmem(n, k, true, kWindowCap) <= limit;
+  p.smem_bytes = WindowSmem(n, k, p.smem_state, kWindowCap);
+  return p.smem_bytes <= limit;
+}
+
+size_t WindowGlobalBytes(int n, int k) { return (size_t)k * WindowLd(n) * 2; }
+
+cudaError_t LaunchDescentWindow(const SmallKPlan& p, const DescentArgs<int16_t>& a, int grid, cudaStream_t st,
+                                bool cfg) {
+  switch (p.k) {
+    case 2: return ByPlacement<2>(p, a, grid, st, cfg);
+    case 3: return ByPlacement<3>(p, a, grid, st, cfg);
+    case 4: return ByPlacement<4>(p, a, grid, st, cfg);
+    case 5: return ByPlacement<5>(p, a, grid, st, cfg);
+    case 6: return ByPlacement<6>(p, a, grid, st, cfg);
+    case 7: return ByPlacement<7>(p, a, grid, st, cfg);
+    case 8: return ByPlacement<8>(p, a, grid, st, cfg);
+    case 16: return ByPlacement<16>(p, a, grid, st, cfg);
+    case 32: return ByPlacement<32>(p, a, grid, st, cfg);
+    case 64: return ByPlacement<64>(p, a, grid, st, cfg);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace ccb

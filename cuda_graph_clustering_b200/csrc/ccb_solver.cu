@@ -225,7 +225,34 @@ bool StreamL2Hints(size_t state_bytes, const Device& dev) {
 // faster (n = 32000, k = 8, pop 128: 608 ms per descent launch in clusters of 4 against 322 ms streamed).
 constexpr bool kClusterDescent = true;
 
-Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop) {
+// Whether the narrow path takes the windowed descent (ccb_descent_window.cuh).  Its windows are long when few vertices
+// share a gain near the best one, so the line is drawn by the width of the gains, about 2.8 sigma with sigma^2 =
+// n p (1 - p) / k the variance of a neighbour count, and the vertices per unit of it (B200, one descent of a slot on
+// G(n, p), us per move, the kernel without windows -> windowed):
+//   k <= 8, at most 1150 vertices a unit:  n = 16000, p = 0.33, k = 3 (190 a unit): 4.5 -> 0.96; n = 32000, p = 0.01,
+//     k = 3 (1110): 5.5 -> 4.6; above it n = 16000, p = 0.01, k = 8 (1280): 4.7 -> 5.5; n = 8000, p = 0.002, k = 3
+//     (1230): 2.5 -> 2.9.  Below n ~ 1280 the bitset fits in shared memory and the register descent needs no row
+//     from L2: n = 1000, p = 0.5, k = 5: 0.42 -> 0.63, against n = 1500, k = 3: 0.68 -> 0.58.
+//   k > 8, at most 2200 a unit:  n = 9001, p = 0.2, k = 24 (230): 11.9 -> 2.9; n = 20000, p = 0.005, k = 9 (2140): 22.9
+//     -> 12.5; up to 1024 vertices all are members and no gain width is needed (n = 1000, p = 0.33, k = 16: 2.2 ->
+//     1.0).  With k > 32 and a width below 4 most keys tie: n = 4000, p = 0.02, k = 64 (width 3.1): 7.5 -> 9.7.
+bool PreferWindow(int n, int k, int64_t edges, bool rows_in_smem) {
+  const double p = n > 1 ? 2.0 * (double)edges / ((double)n * (n - 1)) : 0.0;
+  const double width = 2.8 * std::sqrt(std::max(0.0, n * p * (1.0 - p) / k));
+  if (k <= 8) return !rows_in_smem && n <= 1150.0 * width;
+  return n <= 1024 || (n <= 2200.0 * width && (k <= 32 || width >= 4.0));
+}
+
+// Bytes of the population's descent scratch in global memory (the slots' rows of `next`); 0 when the state is in
+// shared memory or registers.
+size_t NextBytes(const Plan& plan, int n, int k, int ld, int pop) {
+  if (plan.smem_state) return 0;
+  if (plan.sk.window) return (size_t)pop * WindowGlobalBytes(n, k);
+  if (plan.incremental) return (size_t)pop * IncrementalBytes(k, ld);
+  return (size_t)pop * ld * (plan.small_k ? std::max(k, SmallKLanes(k)) : k) * (plan.wide ? 4 : 2);
+}
+
+Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop, int64_t edges) {
   Plan p;
   p.wide = n > CCB_MAX_VERTICES_NARROW || ls_kernel == CCB_LS_WIDE;
   p.threads = DescentThreads(n, p.wide);
@@ -298,6 +325,18 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
     p.smem_rows = false;
     p.threads = sk.threads;
     p.smem_bytes = sk.smem_bytes;
+  }
+  if (!p.wide && k >= 2 && ls_kernel == CCB_LS_AUTO && PreferWindow(n, k, edges, p.small_k && p.sk.smem_rows)) {
+    SmallKPlan w;
+    if (PlanWindow(w, n, k, limit)) {
+      p.sk = w;
+      p.small_k = k <= 8;
+      p.incremental = k > 8;
+      p.smem_state = w.smem_state;
+      p.smem_rows = false;
+      p.threads = w.threads;
+      p.smem_bytes = w.smem_bytes;
+    }
   }
   if (p.wide && (k == 2 || k == 3) && ls_kernel == CCB_LS_AUTO) {
     // one packed word per vertex: the population's state stays in L2
@@ -376,6 +415,7 @@ const char* KernelName(const Plan& p) {
     return p.sparse ? "packed wide k = 2, degree-proportional (per-thread best of each cluster), L2"
                     : "packed wide k = 2 (e = G1 - G0 and the label, 4 bytes per vertex), L2";
   }
+  if (p.sk.window) return p.smem_state ? "windowed, counters in shared memory" : "windowed, counters in L2";
   if (p.incremental && p.wide) return "incremental wide (n <= 65536, uint16 counters, 64-bit keys), L2";
   if (p.incremental) {
     if (p.sk.registers) {
@@ -602,7 +642,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel) {
   s->pop = pop;
   s->ld = std::max(32, (g->n + 31) / 32 * 32);
   s->ls_kernel = ls_kernel;
-  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop);
+  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges);
   // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
   s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
   PlanSmem16(*s);
@@ -610,10 +650,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel) {
   const size_t labels = (size_t)pop * s->ld;
   const size_t gains = labels * k;
   const size_t gb = s->GainBytes();
-  const size_t next_bytes =
-      s->plan.smem_state ? 0
-                         : (s->plan.incremental ? (size_t)pop * IncrementalBytes(k, s->ld)
-                                                : labels * (s->plan.small_k ? std::max(k, SmallKLanes(k)) : k) * gb);
+  const size_t next_bytes = NextBytes(s->plan, g->n, k, s->ld, pop);
   size_t bytes = 2 * labels + gains * gb + next_bytes + (size_t)pop * s->kpad * 4 + 2 * pop * 8 +
                  (size_t)pop * k * g->pitch * 4 + 2 * (size_t)pop * 4 + s->ld + sizeof(Control);
   size_t free_b = 0, total_b = 0;
@@ -627,12 +664,9 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel) {
   uint8_t* cg = nullptr;
   s->Alloc(cg, gains * gb);
   s->cur_g = cg;
-  if (!s->plan.smem_state) {
-    // the global-state descents work in the slot's rows of next: cluster-major G, or packed vectors
-    const size_t bytes_next = s->plan.incremental ? (size_t)pop * IncrementalBytes(k, s->ld)
-                                                  : labels * (s->plan.small_k ? std::max(k, SmallKLanes(k)) : k) * gb;
+  if (next_bytes > 0) {
     uint8_t* ng = nullptr;
-    s->Alloc(ng, bytes_next);
+    s->Alloc(ng, next_bytes);
     s->next_g = ng;
   }
   s->Alloc(s->cur_sizes, (size_t)pop * s->kpad);
@@ -660,6 +694,8 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel) {
   // Shared-memory opt-in for the descent instance of this plan.
   if ((s->plan.incremental && s->plan.wide) || s->plan.packed_wide) {
     // no dynamic shared memory
+  } else if (s->plan.sk.window) {
+    CCB_CUDA(LaunchDescentWindow(s->plan.sk, DescentArgs<int16_t>{}, 0, nullptr, true));
   } else if (s->plan.incremental) {
     CCB_CUDA(LaunchDescentIncremental(s->plan.sk, DescentArgs<int16_t>{}, 0, nullptr, true));
   } else if (s->plan.small_k) {
@@ -754,8 +790,9 @@ void LaunchDescentStep(ccb_solver& s, int grid, int population, int tournament, 
     if (s.plan.small_k || s.plan.incremental) {
       cudaError_t e = cudaSuccess;
       s.timer.Time(kCatDescent, st, [&] {
-        e = s.plan.incremental ? LaunchDescentIncremental(s.plan.sk, a, grid, st, false)
-                               : LaunchDescentSmallK(s.plan.sk, a, grid, st, false);
+        e = s.plan.sk.window   ? LaunchDescentWindow(s.plan.sk, a, grid, st, false)
+            : s.plan.incremental ? LaunchDescentIncremental(s.plan.sk, a, grid, st, false)
+                                 : LaunchDescentSmallK(s.plan.sk, a, grid, st, false);
       });
       CCB_CUDA(e);
       return;
@@ -1115,7 +1152,7 @@ BatchShape ShapeOf(const ccb_solver& s) {
     if ((t.kind >= 0 && t.kind != sh.kind) || s.n < t.n_min || s.n > t.n_max || s.k < t.k_min || s.k > t.k_max) {
       continue;
     }
-    if (t.use_kind == kBatchIncremental && !s.plan.smem_state &&
+    if (t.use_kind == kBatchIncremental && !s.plan.smem_state && !sh.window &&
         (sh.kind == kBatchIncrementalRegs || sh.kind == kBatchIncremental) &&
         (t.threads == 256 || t.threads == 512 || t.threads == 1024)) {
       sh.kind = kBatchIncremental;  // the slot's rows of `next` hold IncrementalBytes: the global-state form fits
@@ -1137,7 +1174,13 @@ BatchShape ShapeOfPlan(const ccb_solver& s) {
   sh.k = s.k;
   sh.threads = sk.threads;
   sh.vpt = sk.vpt;
-  if (s.plan.incremental) {
+  if (sk.window) {  // under the kind its sizes have without it, so that tuning entries find it
+    sh.window = true;
+    sh.kind = s.k <= 8 ? (s.n <= 4096 ? kBatchRegisters : kBatchStream)
+                       : (s.n <= 16384 ? kBatchIncrementalRegs : kBatchIncremental);
+    sh.k = sk.k;
+    sh.smem = sk.smem_state;
+  } else if (s.plan.incremental) {
     sh.kind = sk.registers ? kBatchIncrementalRegs : kBatchIncremental;
     sh.k = 0;
     sh.smem = sk.smem_state;
@@ -1154,6 +1197,7 @@ BatchShape ShapeOfPlan(const ccb_solver& s) {
 
 // Global-memory state bytes per running slot of an L2-streamed bucket (0 when the state is in shared memory).
 size_t L2StateBytes(const ccb_solver& s) {
+  if (s.plan.sk.window) return s.plan.smem_state ? 0 : WindowGlobalBytes(s.n, s.k);
   if (s.plan.incremental) return s.plan.smem_state ? 0 : (s.plan.sk.registers ? (size_t)s.k * s.ld * 2
                                                                                 : IncrementalBytes(s.k, s.ld));
   if (!s.plan.sk.registers && !s.plan.smem_state) return (size_t)s.ld * SmallKLanes(s.k) * 2;
@@ -1169,10 +1213,10 @@ void BuildWorkLists(WorkLists& w, const std::vector<const ccb_solver*>& solvers,
                     double l2_share) {
   w.ReleaseBuckets();
   const int count = (int)solvers.size();
-  std::map<std::tuple<int, int, int, int, int, int, int>, int> index;
+  std::map<std::tuple<int, int, int, int, int, int, int, int>, int> index;
   for (int e = 0; e < count; ++e) {
     const BatchShape sh = ShapeOf(*solvers[e]);
-    const auto key = std::make_tuple(sh.kind, sh.k, sh.threads, sh.vpt, (int)sh.smem, sh.blocks_per_sm, sh.max_slots);
+    const auto key = std::make_tuple((int)sh.window, sh.kind, sh.k, sh.threads, sh.vpt, (int)sh.smem, sh.blocks_per_sm, sh.max_slots);
     auto it = index.find(key);
     if (it == index.end()) {
       it = index.emplace(key, (int)w.buckets.size()).first;
@@ -1242,7 +1286,8 @@ void BuildWorkLists(WorkLists& w, const std::vector<const ccb_solver*>& solvers,
     CCB_CUDA(cudaEventCreateWithFlags(&bk.done, cudaEventDisableTiming));
     char line[200];
     std::snprintf(line, sizeof(line), "%s k=%d threads=%d vpt=%d smem=%d: %zu instances, %d slots, grid %d; ",
-                  bk.shape.kind == kBatchRegisters          ? "registers"
+                  bk.shape.window                           ? "windowed"
+                  : bk.shape.kind == kBatchRegisters        ? "registers"
                   : bk.shape.kind == kBatchStream           ? "stream"
                   : bk.shape.kind == kBatchIncrementalRegs  ? "incremental-registers"
                                                             : "incremental",
@@ -1583,12 +1628,15 @@ size_t RequestBytes(const ccb_server& sv, uint32_t n, const ccb_params& p) {
   const size_t graph = (size_t)std::max<uint32_t>(n, 1) * pitch * 4 + (size_t)std::max<uint32_t>(n, 1) * 4;
   const int ld = std::max(32, ((int)n + 31) / 32 * 32);
   const int kpad = (p.k + 3) / 4 * 4;
-  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population);
+  // The descent, and with it its scratch, depends on the graph's density, not known before a generated graph's
+  // admission: the larger of both.
+  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0);
+  const Plan dense = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population,
+                              (int64_t)n * (n - 1) / 4);
   const size_t labels = (size_t)p.population * ld;
   const size_t gb = plan.wide ? 4 : 2;
-  const size_t next = plan.smem_state ? 0
-                      : plan.incremental ? (size_t)p.population * IncrementalBytes(p.k, ld)
-                                         : labels * (plan.small_k ? std::max(p.k, SmallKLanes(p.k)) : p.k) * gb;
+  const size_t next = std::max(NextBytes(plan, (int)n, p.k, ld, p.population),
+                               NextBytes(dense, (int)n, p.k, ld, p.population));
   return graph + 2 * labels + labels * p.k * gb + next + (size_t)p.population * kpad * 4 + 2 * (size_t)p.population * 8 +
          (size_t)p.population * p.k * pitch * 4 + 2 * (size_t)p.population * 4 + ld + sizeof(Control);
 }
@@ -1706,7 +1754,7 @@ bool BatchedKernelsTake(const ccb_server& sv, const ccb_server::Request& r) {
   const int pitch = std::max(4, (words + 3) / 4 * 4);
   const int ld = std::max(32, ((int)r.n + 31) / 32 * 32);
   const Plan pl = MakePlan((int)r.n, pitch, r.params.k, ld, (r.params.k + 3) / 4 * 4, CCB_LS_AUTO, sv.device,
-                           r.params.population);
+                           r.params.population, 0);
   return !pl.wide && (pl.small_k || pl.incremental);
 }
 
@@ -2249,7 +2297,13 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
   int device = 0;
   CCB_CUDA(cudaGetDevice(&device));
   OneCallCache& c = t_cache;
-  if (c.solver && c.device == device && c.n == n && c.k == k && c.pop == pop && c.ls == ls_kernel) {
+  // the narrow descent depends on the density: another one than the cached solver's needs other buffers
+  const auto same_descent = [&] {
+    const ccb_solver& s = *c.solver;
+    return MakePlan(s.n, s.graph->pitch, k, s.ld, s.kpad, ls_kernel, s.device, pop, (int64_t)edges).sk.window ==
+           s.plan.sk.window;
+  };
+  if (c.solver && c.device == device && c.n == n && c.k == k && c.pop == pop && c.ls == ls_kernel && same_descent()) {
     const int words = (int)((n + 31) / 32);
     if (words_per_row < (uint32_t)words) Fail(CCB_ERR_INVALID, "words_per_row < ceil(n / 32)");
     if (bits == nullptr) Fail(CCB_ERR_INVALID, "null bitset");

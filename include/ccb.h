@@ -209,7 +209,8 @@ typedef struct ccb_tuning_entry {
   int32_t n_min, n_max;  /* inclusive */
   int32_t k_min, k_max;
   int32_t use_kind;      /* -1: the plan's kernel; 2: the incremental kernel with its state in global memory
-                            (taken by kind-2 and kind-3 instances whose state is not in shared memory) */
+                            (taken by kind-2 and kind-3 instances whose state is not in shared memory and that do
+                            not run the windowed descent, which keeps the kind of its sizes) */
   int32_t threads;       /* threads per slot for use_kind 2: 256, 512 or 1024 */
   int32_t blocks_per_sm; /* resident slots per SM of the persistent grid; 0: the occupancy limit */
   int32_t max_slots;     /* cap on the slots running at once (the L2-resident block count); 0: none */
