@@ -148,7 +148,7 @@ __host__ __device__ constexpr uint32_t IdescI8(int m, int n) {
 __device__ __forceinline__ uint32_t Spread4(uint32_t nibble) { return (nibble * 0x00204081u) & 0x01010101u; }
 
 struct TensorArgs {
-  int32_t* g;          // [col][ld], may be null
+  void* g;             // [col][ld] of GainT, may be null
   int ld;
   int n;               // vertices (labels exist for v < n)
   int n_store;         // rows written per column
@@ -164,7 +164,7 @@ struct TensorArgs {
   const Control* stop; // null: always run
 };
 
-template <typename LabelT>
+template <typename LabelT, typename GainT>
 __global__ void __launch_bounds__(kThreads, 1)
     k_rebuild_tensor(const __grid_constant__ CUtensorMap bits_map, const __grid_constant__ CUtensorMap z_map,
                      TensorArgs a) {
@@ -303,37 +303,48 @@ __global__ void __launch_bounds__(kThreads, 1)
     TcFenceAfter();
     const int quarter = warp & 3;
     const LabelT* labels = static_cast<const LabelT*>(a.labels);
+    GainT* g = static_cast<GainT*>(a.g);
     const bool write = ok && !*abort;
     for (int sub = 0; sub < kSubTiles; ++sub) {
       const int v = m0 + sub * kTensorTileM + quarter * kWarp + lane;
       const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * kWarp) << 16) + sub * bn;
-      int cur_slot = -1, own = -1, part = 0;
+      // columns in order: cluster c of slot; a slot's label of v is loaded a slot ahead
+      int slot = n0 / a.k, c = n0 - slot * a.k, part = 0;
+      const int slots = a.columns / a.k;
+      auto label = [&](int of) {
+        return of < slots && v < a.n ? static_cast<int>(labels[static_cast<size_t>(of) * a.label_ld + v]) : -1;
+      };
+      int own = label(slot), own_next = label(slot + 1);
       auto flush = [&]() {
         const unsigned total = __reduce_add_sync(kAllLanes, static_cast<unsigned>(part));
-        if (lane == 0 && write && cur_slot >= 0 && total != 0) {
-          atomicAdd(reinterpret_cast<unsigned long long*>(a.intra + cur_slot), static_cast<unsigned long long>(total));
+        if (lane == 0 && write && total != 0) {
+          atomicAdd(reinterpret_cast<unsigned long long*>(a.intra + slot), static_cast<unsigned long long>(total));
         }
+        part = 0;
       };
+      const bool store = write && g != nullptr && v < a.n_store;
+      GainT* out = g + static_cast<size_t>(n0) * a.ld + v;
       for (int c0 = 0; c0 < bn; c0 += 16) {
+        if (n0 + c0 >= a.columns) break;
         uint32_t acc[16];
         TmemLoad16(lane_addr + c0, acc);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int col = n0 + c0 + i;
-          if (col >= a.columns) break;
-          const int slot = col / a.k;
-          if (slot != cur_slot) {
-            flush();
-            cur_slot = slot;
-            part = 0;
-            own = v < a.n ? static_cast<int>(labels[static_cast<size_t>(slot) * a.label_ld + v]) : -1;
-          }
+          if (n0 + c0 + i >= a.columns) break;
           const int val = static_cast<int>(acc[i]);
-          if (write && a.g != nullptr && v < a.n_store) a.g[static_cast<size_t>(col) * a.ld + v] = val;
-          if (own == col - slot * a.k) part += val;
+          if (store) *out = static_cast<GainT>(val);
+          out += a.ld;
+          part += own == c ? val : 0;
+          if (++c == a.k) {
+            flush();
+            c = 0;
+            ++slot;
+            own = own_next;
+            own_next = label(slot + 1);
+          }
         }
       }
-      flush();
+      if (c != 0) flush();
     }
   }
   TcFenceBefore();
@@ -344,6 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// Z rows, sizes and bad-label flags of the recount's labelings.
 template <typename LabelT>
 __global__ void __launch_bounds__(256)
     k_build_z(const LabelT* __restrict__ labels, int label_ld, int n, int k, int kz, uint8_t* __restrict__ z,
@@ -389,6 +401,74 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The labels of a rebuild (GWW copy, perturbation, neighbourhood or as they are: RebuildBody's first phase), their
+// cluster sizes and their one-hot rows Z in one pass: a block takes `span` vertices of a slot, a thread four of them
+// at a time, whose label bytes and Z words are written whole.
+constexpr int kLabelsThreads = 256;
+template <typename GainT>
+__global__ void __launch_bounds__(kLabelsThreads)
+    k_labels_z(RebuildArgs<GainT> a, uint8_t* __restrict__ z, int kz, int span) {
+  if (a.ctl != nullptr && (a.mode == kRebuildPerturb || a.mode == kRebuildCopy) && a.ctl->stop) return;
+  __shared__ int s_sizes[kMaxK];
+  const int slot = blockIdx.x;
+  const int tid = threadIdx.x;
+  const int lane = tid % kWarp;
+  const int n = a.gr.n, k = a.k, ld = a.ld;
+  for (int c = tid; c < k; c += kLabelsThreads) s_sizes[c] = 0;
+  __syncthreads();
+  const uint8_t* from = a.cur.labels + static_cast<size_t>(slot) * ld;
+  if (a.mode == kRebuildPerturb || a.mode == kRebuildCopy) {
+    from = a.next_labels + static_cast<size_t>(a.src_map != nullptr ? a.src_map[slot] : slot) * ld;
+  }
+  const int center = a.first + slot;
+  const uint32_t* center_row = a.gr.bits + static_cast<size_t>(a.mode == kRebuildNeighborhood ? center : 0) * a.gr.pitch;
+  uint32_t* to = reinterpret_cast<uint32_t*>(a.cur.labels + static_cast<size_t>(slot) * ld);
+  const int words = kz / 4;
+  uint32_t* rows = reinterpret_cast<uint32_t*>(z + static_cast<size_t>(slot) * k * kz);
+  int size0 = 0, size1 = 0;  // of clusters lane and lane + 32
+  const int first = blockIdx.y * span / 4;
+  const int last = min(words, first + span / 4);
+  for (int i = first + tid; i < last; i += kLabelsThreads) {  // whole warps: span is a multiple of 128
+    uint32_t packed = 4 * i < ld && a.mode != kRebuildNeighborhood ? reinterpret_cast<const uint32_t*>(from)[i] : 0u;
+    int l[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int u = 4 * i + j;
+      l[j] = static_cast<int>((packed >> (8 * j)) & 0xffu);
+      if (a.mode == kRebuildNeighborhood) {
+        l[j] = u < n && !(u == center || Bit(center_row, u)) ? 1 : 0;
+      } else if (a.mode == kRebuildPerturb && u < n) {
+        l[j] = PerturbLabelOf(a.stream, static_cast<uint64_t>(slot) * n + u, a.iteration, l[j], k, a.probability);
+      }
+    }
+    packed = static_cast<uint32_t>(l[0]) | static_cast<uint32_t>(l[1]) << 8 | static_cast<uint32_t>(l[2]) << 16 |
+             static_cast<uint32_t>(l[3]) << 24;
+    if (4 * i < n && a.mode != kRebuildInPlace) to[i] = packed;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) l[j] = 4 * i + j < n ? l[j] : -1;
+    for (int c = 0; c < k; ++c) {
+      const uint32_t word = static_cast<uint32_t>(l[0] == c) | static_cast<uint32_t>(l[1] == c) << 8 |
+                            static_cast<uint32_t>(l[2] == c) << 16 | static_cast<uint32_t>(l[3] == c) << 24;
+      rows[static_cast<size_t>(c) * words + i] = word;
+      const int total = __reduce_add_sync(kAllLanes, (word * 0x01010101u) >> 24);
+      size0 += lane == c ? total : 0;
+      size1 += lane + kWarp == c ? total : 0;
+    }
+  }
+  if (lane < k && size0 != 0) atomicAdd(&s_sizes[lane], size0);
+  if (lane + kWarp < k && size1 != 0) atomicAdd(&s_sizes[lane + kWarp], size1);
+  __syncthreads();
+  for (int c = tid; c < k; c += kLabelsThreads) {
+    int32_t* size = a.cur.sizes + static_cast<size_t>(slot) * a.kpad + c;
+    if (gridDim.y == 1) {
+      *size = s_sizes[c];
+    } else if (s_sizes[c] != 0) {
+      atomicAdd(size, s_sizes[c]);
+    }
+  }
+  if (tid == 0 && blockIdx.y == 0) a.intra[slot] = 0;
+}
+
 // f = m + sum_c C(size_c, 2) - intra per labeling (the recount's last step); -1 for a bad label, -2 when the
 // contraction's bounded wait gave up.
 __global__ void k_tensor_finish(const int32_t* sizes, int kpad, const int64_t* intra, const int32_t* bad,
@@ -426,7 +506,7 @@ size_t TensorSmem(int bn) {
 
 }  // namespace
 
-bool PlanTensorRebuild(TensorRebuild& t, int n, int columns, const char** why) {
+bool PlanTensorRebuild(TensorRebuild& t, int n, int columns, int sms, const char** why) {
   if (n < kTensorTileM) {
     *why = "the tensor-core rebuild needs n >= 128";
     return false;
@@ -440,11 +520,23 @@ bool PlanTensorRebuild(TensorRebuild& t, int n, int columns, const char** why) {
   t.ktiles = (t.words + 3) / 4;
   t.kz = t.ktiles * kTileK;
   t.columns = columns;
-  const int blocks = (columns + kTensorMaxN - 1) / kTensorMaxN;
-  t.bn = ((columns + blocks - 1) / blocks + 15) / 16 * 16;
+  t.m_tiles = (n + kTensorTileM * kSubTiles - 1) / (kTensorTileM * kSubTiles);
+  // Columns per CTA: the fewest clocks of the CTAs that one SM runs one after another, by what a CTA was measured to
+  // take: 2400 a K step (expanding 256 rows of bits; the MMAs and the Z copy hide behind it up to 256 columns), 80 a
+  // column of the epilogue.  Wide blocks win when K is long (n = 65536, pop 128, k = 2: one block of 256 columns),
+  // narrow ones fill the SMs when it is short (n = 1000, 2048 columns: 64).
+  long long least = -1;
+  for (int bn = kTensorMaxN; bn >= 16; bn -= 16) {
+    const long long ctas = (long long)t.m_tiles * ((columns + bn - 1) / bn);
+    const long long cost = (ctas + sms - 1) / sms * (2400ll * t.ktiles + 80ll * std::min(bn, columns) + 4000);
+    if (least < 0 || cost < least) {
+      least = cost;
+      t.bn = bn;
+    }
+  }
+  t.bn = std::min(t.bn, (columns + 15) / 16 * 16);
   t.n_tiles = (columns + t.bn - 1) / t.bn;
   t.z_rows = t.n_tiles * t.bn;
-  t.m_tiles = (n + kTensorTileM * kSubTiles - 1) / (kTensorTileM * kSubTiles);
   t.tmem_cols = 32;
   while (t.tmem_cols < kSubTiles * t.bn) t.tmem_cols *= 2;
   t.smem = TensorSmem(t.bn);
@@ -480,22 +572,30 @@ cudaError_t EncodeTensorRebuild(TensorRebuild& t, const uint32_t* bits, int pitc
   return cudaSuccess;
 }
 
-template <typename LabelT>
-cudaError_t LaunchBuildZ(const TensorRebuild& t, const LabelT* labels, int label_ld, int count, int k, int32_t* sizes,
-                         int kpad, int64_t* intra, int32_t* bad, const Control* ctl, cudaStream_t st) {
+template <typename GainT>
+cudaError_t LaunchLabelsZ(const TensorRebuild& t, const RebuildArgs<GainT>& a, int count, int sms, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
-  k_build_z<LabelT><<<count, 256, 0, st>>>(labels, label_ld, t.n, k, t.kz, t.z, sizes, kpad, intra, bad, ctl);
+  // about two blocks per SM, each of whole 128-vertex groups; one block per slot writes the sizes itself
+  const int groups = t.kz / kTileK;
+  const int want = std::max(1, std::min(groups, (2 * sms + count - 1) / count));
+  const int span = (groups + want - 1) / want * kTileK;
+  const int blocks = (t.kz + span - 1) / span;
+  if (blocks > 1) {
+    const cudaError_t e = cudaMemsetAsync(a.cur.sizes, 0, (size_t)count * a.kpad * sizeof(int32_t), st);
+    if (e != cudaSuccess) return e;
+  }
+  k_labels_z<GainT><<<dim3(count, blocks), kLabelsThreads, 0, st>>>(a, t.z, t.kz, span);
   return cudaGetLastError();
 }
 
-template <typename LabelT>
-cudaError_t LaunchTensorRebuild(const TensorRebuild& t, int32_t* g, int ld, int n_store, int count, int k,
+template <typename LabelT, typename GainT>
+cudaError_t LaunchTensorRebuild(const TensorRebuild& t, GainT* g, int ld, int n_store, int count, int k,
                                 const LabelT* labels, int label_ld, int64_t* intra, int32_t* error, const Control* ctl,
                                 cudaStream_t st) {
   const int columns = count * k;
   if (columns <= 0) return cudaSuccess;
   if (columns > t.z_rows) return cudaErrorInvalidValue;
-  const cudaError_t attr = cudaFuncSetAttribute(k_rebuild_tensor<LabelT>,
+  const cudaError_t attr = cudaFuncSetAttribute(k_rebuild_tensor<LabelT, GainT>,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem);
   if (attr != cudaSuccess) return attr;
   TensorArgs a{};
@@ -514,14 +614,18 @@ cudaError_t LaunchTensorRebuild(const TensorRebuild& t, int32_t* g, int ld, int 
   a.error = error;
   a.stop = ctl;
   const dim3 grid(t.m_tiles, (columns + t.bn - 1) / t.bn);
-  k_rebuild_tensor<LabelT><<<grid, kThreads, t.smem, st>>>(t.bits_map, t.z_map, a);
+  k_rebuild_tensor<LabelT, GainT><<<grid, kThreads, t.smem, st>>>(t.bits_map, t.z_map, a);
   return cudaGetLastError();
 }
 
-template cudaError_t LaunchBuildZ<uint8_t>(const TensorRebuild&, const uint8_t*, int, int, int, int32_t*, int, int64_t*,
-                                           int32_t*, const Control*, cudaStream_t);
-template cudaError_t LaunchTensorRebuild<uint8_t>(const TensorRebuild&, int32_t*, int, int, int, int, const uint8_t*,
-                                                  int, int64_t*, int32_t*, const Control*, cudaStream_t);
+template cudaError_t LaunchLabelsZ<int16_t>(const TensorRebuild&, const RebuildArgs<int16_t>&, int, int, cudaStream_t);
+template cudaError_t LaunchLabelsZ<int32_t>(const TensorRebuild&, const RebuildArgs<int32_t>&, int, int, cudaStream_t);
+template cudaError_t LaunchTensorRebuild<uint8_t, int16_t>(const TensorRebuild&, int16_t*, int, int, int, int,
+                                                           const uint8_t*, int, int64_t*, int32_t*, const Control*,
+                                                           cudaStream_t);
+template cudaError_t LaunchTensorRebuild<uint8_t, int32_t>(const TensorRebuild&, int32_t*, int, int, int, int,
+                                                           const uint8_t*, int, int64_t*, int32_t*, const Control*,
+                                                           cudaStream_t);
 
 }  // namespace ccb
 
@@ -548,14 +652,18 @@ int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t wor
   if ((long long)count * k > (1 << 24)) return report(CCB_ERR_INVALID, "count * k exceeds 16777216");
   TensorRebuild t;
   const char* why = nullptr;
-  if (!PlanTensorRebuild(t, (int)n, count * k, &why)) return report(CCB_ERR_INVALID, why);
+  int device = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return report(CCB_ERR_CUDA, cudaGetErrorString(e));
+  if (!PlanTensorRebuild(t, (int)n, count * k, sms, &why)) return report(CCB_ERR_INVALID, why);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int kpad = (k + 3) / 4 * 4;
   const size_t z_bytes = (size_t)t.z_rows * t.kz;
   const size_t sizes_bytes = sizes_out ? 0 : (size_t)count * kpad * 4;
   const size_t scratch = z_bytes + (size_t)count * 8 + (size_t)count * 4 + 16 + sizes_bytes;
   uint8_t* buf = nullptr;
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&buf), scratch, st);
+  e = cudaMallocAsync(reinterpret_cast<void**>(&buf), scratch, st);
   if (e != cudaSuccess) return report(CCB_ERR_DEVICE_MEMORY, cudaGetErrorString(e));
   uint8_t* z = buf;
   int64_t* intra = reinterpret_cast<int64_t*>(buf + z_bytes);  // z_bytes is a multiple of 128
@@ -575,7 +683,7 @@ int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t wor
   const int label_ld = (int)n;
   k_build_z<int32_t><<<count, 256, 0, st>>>(labels, label_ld, (int)n, k, t.kz, z, sizes, sizes_ld, intra, bad, nullptr);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
-  if ((e = LaunchTensorRebuild<int32_t>(t, g_out, (int)n, (int)n, count, k, labels, label_ld, intra, error, nullptr,
+  if ((e = LaunchTensorRebuild<int32_t, int32_t>(t, g_out, (int)n, (int)n, count, k, labels, label_ld, intra, error, nullptr,
                                         st)) != cudaSuccess) {
     return fail(e);
   }

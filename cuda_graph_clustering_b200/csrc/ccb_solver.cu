@@ -514,6 +514,7 @@ struct ccb_solver {
   uint32_t* masks = nullptr;
   int64_t* intra = nullptr;    // tiled rebuild (wide path): per-slot intra-cluster sums; null: per-slot rebuild
   int rebuild_kind = CCB_REBUILD_AUTO;
+  bool plain = true;  // iterated by the plain path's kernels (false: by the batched engine's, which rebuild by popcount)
   std::unique_ptr<TensorRebuild> tensor;  // set: the wide path rebuilds G on the tensor cores
   int32_t* src_map = nullptr;
   int32_t* order = nullptr;
@@ -586,7 +587,8 @@ void Describe(ccb_solver& s) {
   const size_t smem = s.plan.smem16 ? (s.k == 2 ? Wide2Smem16Bytes(s.n) : Wide3Smem26Bytes(s.n)) : s.plan.smem_bytes;
   std::snprintf(text, sizeof(text), "%s, %d threads per block, %d blocks, %zu bytes of shared memory%s",
                 KernelName(s.plan), s.plan.threads, s.pop * std::max(1, s.plan.sk.cluster), smem,
-                s.tensor ? "; G rebuilt on the tensor cores (int8 tcgen05, TMA)" : "");
+                !s.tensor ? "" : s.plan.wide ? "; G rebuilt on the tensor cores (int8 tcgen05, TMA)"
+                                             : "; G rebuilt by an int8 tcgen05 contraction");
   s.description = text;
 }
 
@@ -594,14 +596,24 @@ void Describe(ccb_solver& s) {
 // phase of a 50-iteration solve takes 83 ms at k = 2 and 125 ms at k = 3, against 412 / 654 ms by popcount).
 constexpr bool kTensorRebuildByDefault = true;
 
+// Whether CCB_REBUILD_AUTO takes the tensor cores on the narrow path: its three launches cost about 28 us, the popcount
+// rebuild (one slot per block) grows with the words it intersects.  us a rebuild, popcount -> tensor (B200, pop 128):
+// n = 1000, k = 5 (128K words a slot) 21 -> 32; n = 700, k = 16 (231K) 33 -> 32; n = 1000, k = 16 (480K) 46 -> 34; n =
+// 2000, k = 32 282 -> 65; n = 16000, k = 3 1902 -> 160; n = 32000, k = 8 13650 -> 988.
+bool PreferTensorNarrow(const ccb_solver& s) {
+  return s.n >= 128 && (long long)s.n * s.graph->words * (s.k - 1) >= 250000;
+}
+
 // Whether the solver rebuilds G on the tensor cores: the tiled wide rebuild (int32 G) with n >= 128, chosen
 // explicitly or by CCB_REBUILD_AUTO.
 bool WantTensor(const ccb_solver& s, int kind) {
-  if (s.intra == nullptr || kind == CCB_REBUILD_POPCOUNT) return false;
+  if (kind == CCB_REBUILD_POPCOUNT) return false;
+  if (!s.plan.wide) return kind == CCB_REBUILD_AUTO && s.plain && PreferTensorNarrow(s);
+  if (s.intra == nullptr) return false;
   if (kind == CCB_REBUILD_AUTO && !kTensorRebuildByDefault) return false;
   TensorRebuild t;
   const char* why = nullptr;
-  return PlanTensorRebuild(t, s.n, s.pop * s.k, &why);
+  return PlanTensorRebuild(t, s.n, s.pop * s.k, s.device.sms, &why);
 }
 
 // Sets the rebuild kind; allocates the one-hot buffer and encodes the tensor maps when the tensor path is on.
@@ -621,7 +633,13 @@ void SetRebuild(ccb_solver& s, int kind) {
   if (s.tensor) return;
   std::unique_ptr<TensorRebuild> t(new TensorRebuild());
   const char* why = nullptr;
-  PlanTensorRebuild(*t, s.n, s.pop * s.k, &why);
+  PlanTensorRebuild(*t, s.n, s.pop * s.k, s.device.sms, &why);
+  if (!s.plan.wide) {  // the popcount rebuild where Z would take memory the caller may count on
+    size_t free_b = 0, total_b = 0;
+    CCB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if ((size_t)t->z_rows * t->kz > free_b / 4) return;
+    if (s.intra == nullptr) s.Alloc(s.intra, s.pop);
+  }
   uint8_t* z = nullptr;
   s.Alloc(z, (size_t)t->z_rows * t->kz);
   CCB_CUDA(cudaMemset(z, 0, (size_t)t->z_rows * t->kz));
@@ -630,7 +648,7 @@ void SetRebuild(ccb_solver& s, int kind) {
   s.tensor = std::move(t);
 }
 
-ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel) {
+ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool plain = true) {
   TraceRange trace_range("ccb.solver.create");
   std::unique_ptr<ccb_solver> s(new ccb_solver());
   s->graph = g;
@@ -642,6 +660,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel) {
   s->pop = pop;
   s->ld = std::max(32, (g->n + 31) / 32 * 32);
   s->ls_kernel = ls_kernel;
+  s->plain = plain;
   s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges);
   // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
   s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
@@ -728,6 +747,26 @@ void LaunchRebuild(ccb_solver& s, int grid, int mode, const int32_t* src_map, ui
   const Control* ctl = check_stop ? s.ctl : nullptr;
   RebuildArgs<GainT> a{s.graph->View(), s.Cur<GainT>(), s.next_lab, src_map, s.masks, s.k, s.kpad, s.ld,
                        mode, stream, iteration, prob, first, ctl};
+  if (s.tensor) {  // labels, sizes and Z; the tensor-core contraction; f
+    a.intra = s.intra;
+    const Control* stop = (mode == kRebuildPerturb || mode == kRebuildCopy) ? ctl : nullptr;
+    int32_t* error = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(s.ctl) + offsetof(Control, error));
+    cudaError_t e = cudaSuccess;
+    s.timer.Time(kCatRebuild, st, [&] {
+      e = LaunchLabelsZ<GainT>(*s.tensor, a, grid, s.device.sms, st);
+      if (e == cudaSuccess) {
+        e = LaunchTensorRebuild<uint8_t, GainT>(*s.tensor, s.Cur<GainT>().g, s.ld, s.n, grid, s.k, s.cur_lab, s.ld,
+                                                s.intra, error, stop, st);
+      }
+      if (e == cudaSuccess) {
+        k_rebuild_finish<GainT><<<(grid + 127) / 128, 128, 0, st>>>(s.Cur<GainT>(), s.intra, grid, s.k, s.kpad,
+                                                                    (int64_t)s.graph->edges, mode, ctl);
+      }
+    });
+    CCB_CUDA(e);
+    CCB_CUDA(cudaGetLastError());
+    return;
+  }
   if constexpr (std::is_same_v<GainT, int32_t>) {
     if (s.intra != nullptr) {
       a.intra = s.intra;
@@ -735,27 +774,6 @@ void LaunchRebuild(ccb_solver& s, int grid, int mode, const int32_t* src_map, ui
       const RebuildTilesArgs t{g.View(), s.cur_lab, s.masks, s.Cur<int32_t>().g, s.intra, grid, s.k, s.ld, mode, ctl};
       const int tiles = (g.n + kRebuildTileThreads / kWarp - 1) / (kRebuildTileThreads / kWarp);
       const size_t smem = (size_t)kRebuildTileThreads / kWarp * g.pitch * 4;
-      if (s.tensor) {
-        // labels, masks and sizes as above; then Z, the tensor-core contraction and f
-        const Control* stop = (mode == kRebuildPerturb || mode == kRebuildCopy) ? ctl : nullptr;
-        int32_t* error = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(s.ctl) + offsetof(Control, error));
-        cudaError_t e = cudaSuccess;
-        s.timer.Time(kCatRebuild, st, [&] {
-          k_rebuild<GainT, kRebuildThreads><<<grid, kRebuildThreads, 0, st>>>(a);
-          e = LaunchBuildZ<uint8_t>(*s.tensor, s.cur_lab, s.ld, grid, s.k, nullptr, 0, nullptr, nullptr, stop, st);
-          if (e == cudaSuccess) {
-            e = LaunchTensorRebuild<uint8_t>(*s.tensor, s.Cur<int32_t>().g, s.ld, g.n, grid, s.k, s.cur_lab, s.ld,
-                                             s.intra, error, stop, st);
-          }
-          if (e == cudaSuccess) {
-            k_rebuild_finish<GainT><<<(grid + 127) / 128, 128, 0, st>>>(s.Cur<GainT>(), s.intra, grid, s.k, s.kpad,
-                                                                        (int64_t)g.edges, mode, ctl);
-          }
-        });
-        CCB_CUDA(e);
-        CCB_CUDA(cudaGetLastError());
-        return;
-      }
       s.timer.Time(kCatRebuild, st, [&] {
         k_rebuild<GainT, kRebuildThreads><<<grid, kRebuildThreads, 0, st>>>(a);
         k_rebuild_tiles<kRebuildTileThreads><<<tiles, kRebuildTileThreads, smem, st>>>(t);
@@ -1343,7 +1361,7 @@ void PrepareBatch(ccb_batch& b) {
   for (size_t i = 0; i < b.inst.size(); ++i) {
     ccb_batch::Instance& in = b.inst[i];
     if (in.graph->n == 0) continue;
-    in.solver.reset(MakeSolver(in.graph, in.params.k, in.params.population, CCB_LS_AUTO));
+    in.solver.reset(MakeSolver(in.graph, in.params.k, in.params.population, CCB_LS_AUTO, false));
     const Plan& pl = in.solver->plan;
     in.batched = !pl.wide && (pl.small_k || pl.incremental);
     if (!in.batched) continue;
@@ -1792,7 +1810,7 @@ void Admit(ccb_server& sv) {
         Finish(sv, a, r0, {});
         continue;
       }
-      a.solver.reset(MakeSolver(a.graph.get(), q.params.k, q.params.population, CCB_LS_AUTO));
+      a.solver.reset(MakeSolver(a.graph.get(), q.params.k, q.params.population, CCB_LS_AUTO, false));
       const Plan& pl = a.solver->plan;
       if (pl.wide || !(pl.small_k || pl.incremental)) {
         CCB_CUDA(cudaStreamSynchronize(sv.stream));  // the graph is complete before another stream reads it

@@ -110,3 +110,33 @@ def test_tensor_rebuild_matches_the_reference_binary_at_65536(ccb, cuda_device, 
     assert (got.objective, got.iterations_done, got.clusters_used) == \
         (run["objective"], run["iterations_done"], run["clusters_used"])
     assert hashlib.sha256(np.asarray(got.labels, dtype="<i4").tobytes()).hexdigest() == run["labels_sha256"]
+
+
+# The narrow path's tensor rebuild (int16 G, taken by size): the line that selects it, ragged n, column blocks that end
+# inside a slot, populations of one block per slot and of several, the Neighborhood's last partial batch.
+@pytest.mark.parametrize("n,k,pop,density", [(707, 16, 5, 0.3), (730, 16, 40, 0.3), (1001, 64, 7, 0.5),
+                                             (1409, 17, 150, 0.2), (4100, 3, 3, 0.3), (2049, 33, 20, 0.1)])
+def test_narrow_rebuild_matches_oracle(ccb, oracle, cuda_device, n, k, pop, density):
+    bits, edges = oracle.erdos_renyi(n, density, n + k)
+    p = dict(k=k, population=pop, iterations=2, early_stop=10, gww=0.25, seed=5)
+    g = ccb.DeviceGraph(ccb.Graph(n, bits, edges))
+    s = ccb.Solver(g, ccb.PbilsParams(**p))
+    assert ("tcgen05" in s.describe()) == (n * ((n + 31) // 32) * (k - 1) >= 250000)
+    want = oracle.pbils(bits, edges, make_params(**p))
+    for kind in ("auto", "popcount", "auto"):
+        s.set_rebuild(kind)
+        got = s.pbils(ccb.PbilsParams(**p))
+        assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves), kind
+        assert np.array_equal(got.labels, want.labels), kind
+
+
+@pytest.mark.parametrize("local_search", [False, True])
+def test_narrow_neighborhood_rebuild_matches_oracle(ccb, oracle, cuda_device, local_search):
+    bits, edges, _ = oracle.planted(2900, 2, True, 0.6, 0.1, 0.0, 4)
+    s = ccb.Solver(ccb.DeviceGraph(ccb.Graph(2900, bits, edges)), ccb.PbilsParams(k=2, population=120))
+    assert "tcgen05" in s.describe()
+    got = s.neighborhood(ccb.PbilsParams(k=2, population=120), local_search)
+    s.set_rebuild("popcount")
+    want = s.neighborhood(ccb.PbilsParams(k=2, population=120), local_search)
+    assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+    assert np.array_equal(got.labels, want.labels)
