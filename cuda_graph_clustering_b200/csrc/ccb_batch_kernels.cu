@@ -356,7 +356,7 @@ cudaError_t WithKernel(const BatchShape& s, F&& f) {
     if (s.smem) { CCB_PICK((kb_descent_registers<K, T, V, true>), (kf_registers<K, T, V, true>)) }     \
     CCB_PICK((kb_descent_registers<K, T, V, false>), (kf_registers<K, T, V, false>))                   \
   }
-#define CCB_REG_K(K) CCB_REG(K, 128, 4) CCB_REG(K, 256, 4) CCB_REG(K, 512, 4) CCB_REG(K, 1024, 4)
+#define CCB_REG_K(K) CCB_REG(K, 64, 4) CCB_REG(K, 128, 8) CCB_REG(K, 128, 4) CCB_REG(K, 256, 4) CCB_REG(K, 512, 4) CCB_REG(K, 1024, 4)
   CCB_REG_K(2) CCB_REG_K(3) CCB_REG_K(4) CCB_REG_K(5) CCB_REG_K(6) CCB_REG_K(7) CCB_REG_K(8)
 #undef CCB_REG_K
 #undef CCB_REG

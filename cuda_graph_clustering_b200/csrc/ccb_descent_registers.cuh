@@ -42,58 +42,37 @@ __device__ __forceinline__ void LanesMinMax(const int* x, int& lo, int& hi) {
   }
 }
 
-// ---- compact keys (n <= 1023) ---------------------------------------------------------------------------
-// With B = bit width of n <= 10 and S = B + 8, a vertex's lanes are
-//     foreign c:  L_c = (h_c << S) + c          own a:  L_a = ((h_a + P) << S) - 16 a,    P = 2^(B+1)
-// (|h| <= n < 2^B, so every foreign lane is below 2^(B+S) and the own lane above it: max = own, min = the best
-// foreign target, smaller cluster first).  Then the block's move key of the vertex is a single add:
-//     kmin - kmax + ((P + 1 + 2^B) << S) + (u << 8) = ((gain + 2^B) << S) | (u << 8) | (a << 4) | to,
-// gain + 2^B in [2, 2^(B+1)) since the gain is in [1 - n, n - 1]: smaller gain, then smaller vertex, as the
-// reference orders moves, with both clusters riding in the low byte.  A move (v: from -> to) changes lanes
-// `from` and `to` of every vertex by -/+ 2^S (sign by adjacency to v), folded into the next scan.  Keys are
-// unsigned so that the lanes of absent vertices (u >= n, ignored) wrap instead of overflowing.
+// ---- compact pairs (n <= 1023) --------------------------------------------------------------------------
+// Two vertices share 32-bit registers, a 16-bit lane each.  A vertex's K lanes are
+//     foreign c:  8 (h_c + 1024) + c  (below 2^14, |h| <= n)      own a:  the same + 2^15,
+// so that over the lanes the minimum is the best foreign target (smaller cluster first) and the maximum the own
+// cluster.  Thread t holds the pairs (2 q, 2 q + 1), q = t + p T: their bits lie side by side in one row word.  A move
+// (v: from -> to) adds +-8 to lanes `from` and -+8 to lanes `to` of every vertex by adjacency to v: with d the packed
+// pair of +-8, one multiply-add of the 32-bit register per lane (no half leaves [0, 2^16), so none carries into the
+// other).  The gain field of a vertex is X = (min & ~7) - (max & ~7) + 0xC000 = 8 (gain - 1) + 2^14; its move key
+// X << 16 | u << 6 | from << 3 | to orders by gain, then vertex, and carries both clusters.  Lanes of absent vertices
+// never move (no adjacency, no -8) and hold a gain that is never chosen.
+//
+// Bound by issue: 32-bit adds and multiply-adds take two clocks a warp here, 16-bit pair minima one, and every warp
+// pays the move's overhead (argmin, decode, row address), so 128 threads hold 8 vertices each.  ns a move of 128 slots
+// (B200), with one 32-bit key a lane on 256 threads and now: n = 1000, p = 0.5, k = 5 416, 279 (64 threads x 16: 415,
+// 256 x 4: 336); n = 500, k = 8 456, 270; n = 200, k = 4 455, 304.
 constexpr int kCompactMaxBits = 10;
-
-// One scan of the vertices: fold the last move into lanes (coef[c] = [c = from] - [c = to] times the signed step,
-// by adjacency to the moved vertex), then each vertex's move key.
-template <int K, int V>
-__device__ __forceinline__ uint32_t CompactScan(uint32_t (&key)[V][K], const uint32_t (&rw)[V], uint32_t lane_bit,
-                                                const uint32_t (&cu)[V], unsigned valid, const int (&coef)[K],
-                                                int step) {
-  uint32_t best = ~0u;
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const int d = (rw[j] & lane_bit) ? step : -step;
-    int lanes[K];
-#pragma unroll
-    for (int c = 0; c < K; ++c) {
-      key[j][c] += static_cast<uint32_t>(coef[c] * d);
-      lanes[c] = static_cast<int>(key[j][c]);
-    }
-    int kmin, kmax;
-    LanesMinMax<K>(lanes, kmin, kmax);
-    const uint32_t mk = static_cast<uint32_t>(kmin - kmax) + cu[j];
-    best = min(best, ((valid >> j) & 1) ? mk : ~0u);
-  }
-  return best;
-}
 
 template <int K, int T, int V>
 __device__ __forceinline__ void DescentRegistersCompact(const DescentArgs<int16_t>& a, int slot, int w,
-                                                        const uint32_t* rows, MoveRecord<uint32_t>* s_records) {
+                                                        const uint32_t* rows, uint32_t* s_records) {
   constexpr int kWarps = T / kWarp;
+  constexpr int P = V / 2;
+  constexpr uint32_t kClusterBits = 0x00070007u;
   const int tid = threadIdx.x;
   const int lane = tid % kWarp;
   const int n = a.gr.n;
   const int ld = a.ld;
-  const int bits = a.key_bits;
-  const int shift = bits + 8;
-  const uint32_t step = 1u << shift;
-  const uint32_t penalty = (2u << bits) << shift;
 
-  uint32_t key[V][K];
-  uint32_t cu[V];
-  unsigned valid = 0;
+  uint32_t key[P][K];
+  uint32_t code[P];  // u << 6 of both vertices
+  uint32_t down[P];  // 8 in the half of each present vertex
   {
     const int16_t* g_src = a.cur.g + static_cast<size_t>(w) * K * ld;
     const uint8_t* l_src = a.cur.labels + static_cast<size_t>(w) * ld;
@@ -101,86 +80,111 @@ __device__ __forceinline__ void DescentRegistersCompact(const DescentArgs<int16_
     int sz[K];
 #pragma unroll
     for (int c = 0; c < K; ++c) sz[c] = sizes[c];
-    const uint32_t base = ((2u << bits) + 1u + (1u << bits)) << shift;
 #pragma unroll
-    for (int j = 0; j < V; ++j) {
-      const int u = tid + j * T;
-      const bool ok = u < n;
-      valid |= ok ? (1u << j) : 0u;
-      const int own = ok ? l_src[u] : 0;
+    for (int p = 0; p < P; ++p) {
+      code[p] = 0u;
+      down[p] = 0u;
 #pragma unroll
-      for (int c = 0; c < K; ++c) {
-        const int h = sz[c] - 2 * (ok ? static_cast<int>(g_src[static_cast<size_t>(c) * ld + u]) : 0);
-        const uint32_t lane_key = (static_cast<uint32_t>(h) << shift) + static_cast<uint32_t>(c);
-        key[j][c] = c == own ? lane_key + penalty - 17u * static_cast<uint32_t>(c) : lane_key;
-      }
-      cu[j] = base + (static_cast<uint32_t>(ok ? u : 0) << 8);
-    }
-  }
-  long long objective = a.cur.f[w];
-  const long long move_budget = objective;
-  unsigned long long applied = 0;
-  int parity = 0;
-  const uint32_t lane_bit = 1u << lane;
-  const uint32_t no_move = (1u << bits) << shift;
-  const uint32_t vmask = (1u << bits) - 1u;
-
-  uint32_t rw[V];
-  int coef[K];
+      for (int c = 0; c < K; ++c) key[p][c] = 0u;
 #pragma unroll
-  for (int j = 0; j < V; ++j) rw[j] = 0u;
+      for (int half = 0; half < 2; ++half) {
+        const int u = 2 * (tid + p * T) + half;
+        const bool ok = u < n;
+        const int own = ok ? l_src[u] : 0;
+        code[p] |= static_cast<uint32_t>(ok ? u << 6 : 0) << (16 * half);
+        down[p] |= (ok ? 8u : 0u) << (16 * half);
 #pragma unroll
-  for (int c = 0; c < K; ++c) coef[c] = 0;
-  uint32_t best = CompactScan<K, V>(key, rw, lane_bit, cu, valid, coef, static_cast<int>(step));
-  while (true) {
-    const uint32_t mkey = BlockArgMin<uint32_t, kWarps>(best, 0u, s_records + parity * kWarps).key;
-    if (mkey >= no_move) break;
-    parity ^= 1;
-    const int v = static_cast<int>((mkey >> 8) & vmask);
-    const int from = static_cast<int>((mkey >> 4) & 15u);
-    const int to = static_cast<int>(mkey & 15u);
-    if ((v % T) == tid) {  // the moved vertex's own lane moves from `from` to `to`
-      const int jv = v / T;
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        if (j == jv) {
-#pragma unroll
-          for (int c = 0; c < K; ++c) {
-            if (c == from) key[j][c] += 17u * static_cast<uint32_t>(c) - penalty;
-            if (c == to) key[j][c] += penalty - 17u * static_cast<uint32_t>(c);
-          }
+        for (int c = 0; c < K; ++c) {
+          const int h = ok ? sz[c] - 2 * static_cast<int>(g_src[static_cast<size_t>(c) * ld + u]) : (c == 0 ? -1024 : 1023);
+          key[p][c] |= static_cast<uint32_t>(8 * (h + 1024) + c + (c == own ? 0x8000 : 0)) << (16 * half);
         }
       }
     }
-    objective += static_cast<long long>(static_cast<int>(mkey >> shift) - (1 << bits));
-    ++applied;
-    if (static_cast<long long>(applied) > move_budget) {
+  }
+  const long long start = a.cur.f[w];
+  const int move_budget = static_cast<int>(start);  // f <= n (n - 1) / 2: every move lowers it
+  int gained = 0;
+  int applied = 0;
+  int from = 0, to = 0;
+  int mine = -1;          // the moved vertex's pair among this thread's
+  uint32_t bias = 0u;     // the own-cluster bias in the moved vertex's half
+  const int shift = 2 * (tid & 15);
+  const uint32_t* row = nullptr;
+
+  while (true) {
+    if (row != nullptr) {  // fold the last move into the lanes
+      uint32_t rw[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) rw[p] = 2 * (tid + p * T) < n ? row[(tid + p * T) >> 4] : 0u;
+      int coef[K];
+#pragma unroll
+      for (int c = 0; c < K; ++c) coef[c] = (c == from ? 1 : 0) - (c == to ? 1 : 0);
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const uint32_t y = rw[p] >> shift;
+        const uint32_t bits = (y & 1u) | ((y << 15) & 0x10000u);
+        const int d = static_cast<int>(bits * 16u - down[p] - (mine == p ? bias : 0u));
+#pragma unroll
+        for (int c = 0; c < K; ++c) key[p][c] += static_cast<uint32_t>(coef[c] * d);
+      }
+    }
+    uint32_t best = ~0u;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      uint32_t lo = key[p][0], hi = key[p][0];
+#pragma unroll
+      for (int c = 1; c < K; ++c) {
+        lo = __vminu2(lo, key[p][c]);
+        hi = __vmaxu2(hi, key[p][c]);
+      }
+      const uint32_t x = (lo & ~kClusterBits) - (hi & ~kClusterBits) + 0xC000C000u;
+      const uint32_t low = code[p] | (lo & kClusterBits) | ((hi << 3) & (kClusterBits << 3));
+      best = min(best, min(__byte_perm(low, x, 0x5410), __byte_perm(low, x, 0x7632)));
+    }
+    // the block's best key: each warp's to shared memory (double-buffered), one barrier
+    best = WarpMin(best);
+    if constexpr (kWarps > 1) {
+      uint32_t* rec = s_records + (applied & 1) * kWarps;
+      if (lane == 0) rec[tid / kWarp] = best;
+      __syncthreads();
+      if constexpr (kWarps == 2) {
+        const uint2 r = *reinterpret_cast<const uint2*>(rec);
+        best = min(r.x, r.y);
+      } else if constexpr (kWarps == 4) {
+        const uint4 r = *reinterpret_cast<const uint4*>(rec);
+        best = min(min(r.x, r.y), min(r.z, r.w));
+      } else {
+        best = WarpMin(lane < kWarps ? rec[lane] : ~0u);
+      }
+    }
+    if (best >= (16384u - 8u) << 16) break;  // gain >= 0
+    const int v = static_cast<int>((best >> 6) & 1023u);
+    from = static_cast<int>((best >> 3) & 7u);
+    to = static_cast<int>(best & 7u);
+    row = rows + v * a.gr.pitch;
+    const int q = v >> 1;
+    mine = q % T == tid ? q / T : -1;
+    bias = 0x8000u << (16 * (v & 1));
+    gained += (static_cast<int>(best >> 16) - 16384) / 8 + 1;
+    if (++applied > move_budget) {
       if (tid == 0) atomicExch(&a.ctl->error, kErrorMoveBound);
       break;
     }
-    const uint32_t* row = rows + static_cast<size_t>(v) * a.gr.pitch;
-#pragma unroll
-    for (int j = 0; j < V; ++j) rw[j] = ((valid >> j) & 1) ? row[(tid + j * T) >> 5] : 0u;  // words < ceil(n/32)
-#pragma unroll
-    for (int c = 0; c < K; ++c) coef[c] = (c == from ? 1 : 0) - (c == to ? 1 : 0);
-    best = CompactScan<K, V>(key, rw, lane_bit, cu, valid, coef, static_cast<int>(step));
   }
 
   uint8_t* dst = a.next.labels + static_cast<size_t>(slot) * ld;
 #pragma unroll
-  for (int j = 0; j < V; ++j) {
-    if ((valid >> j) & 1) {
-      int lanes[K];
+  for (int p = 0; p < P; ++p) {
+    uint32_t hi = key[p][0];
 #pragma unroll
-      for (int c = 0; c < K; ++c) lanes[c] = static_cast<int>(key[j][c]);
-      int kmin, kmax;
-      LanesMinMax<K>(lanes, kmin, kmax);
-      dst[tid + j * T] = static_cast<uint8_t>(((0u - static_cast<uint32_t>(kmax)) >> 4) & 15u);
-    }
+    for (int c = 1; c < K; ++c) hi = __vmaxu2(hi, key[p][c]);
+    const int u = 2 * (tid + p * T);
+    if (u < n) dst[u] = static_cast<uint8_t>(hi & 7u);
+    if (u + 1 < n) dst[u + 1] = static_cast<uint8_t>((hi >> 16) & 7u);
   }
   if (tid == 0) {
-    a.next.f[slot] = objective;
-    if (applied) atomicAdd(&a.ctl->moves, applied);
+    a.next.f[slot] = start + gained;
+    if (applied) atomicAdd(&a.ctl->moves, static_cast<unsigned long long>(applied));
   }
 }
 
@@ -190,7 +194,7 @@ __device__ __forceinline__ void DescentRegisters(const DescentArgs<int16_t>& a, 
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_winner;
   __shared__ int s_stop;
-  __shared__ MoveRecord<uint32_t> s_records[2 * kWarps];
+  __shared__ __align__(16) MoveRecord<uint32_t> s_records[2 * kWarps];
 
   const int tid = threadIdx.x;
   const int lane = tid % kWarp;
@@ -220,7 +224,7 @@ __device__ __forceinline__ void DescentRegisters(const DescentArgs<int16_t>& a, 
   const int w = s_winner;
   if constexpr (T * V <= 1024) {
     if (a.key_bits <= kCompactMaxBits) {
-      DescentRegistersCompact<K, T, V>(a, slot, w, rows, s_records);
+      DescentRegistersCompact<K, T, V>(a, slot, w, rows, reinterpret_cast<uint32_t*>(s_records));
       return;
     }
   }

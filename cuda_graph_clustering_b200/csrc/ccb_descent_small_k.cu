@@ -48,6 +48,7 @@ cudaError_t RegistersByShape(int threads, int vpt, const DescentArgs<int16_t>& a
     }
   }
   switch (threads) {
+    case 64: return GoRegisters<K, 64, 4, R>(a, grid, smem, st, cfg);
     case 128: return GoRegisters<K, 128, 4, R>(a, grid, smem, st, cfg);
     case 256: return GoRegisters<K, 256, 4, R>(a, grid, smem, st, cfg);
     case 512: return GoRegisters<K, 512, 4, R>(a, grid, smem, st, cfg);
@@ -171,7 +172,7 @@ size_t RegistersSmem(int n, int pitch, bool smem_rows) {
 
 bool RegistersShapeBuilt(int threads, int vpt) {
   return (vpt == 16 && threads == 64) || (vpt == 8 && (threads == 128 || threads == 256 || threads == 512)) ||
-         (vpt == 4 && (threads == 128 || threads == 256 || threads == 512 || threads == 1024));
+         (vpt == 4 && (threads == 64 || threads == 128 || threads == 256 || threads == 512 || threads == 1024));
 }
 
 cudaError_t LaunchDescentSmallK(const SmallKPlan& p, const DescentArgs<int16_t>& a, int grid, cudaStream_t st,

@@ -171,13 +171,22 @@ struct Plan {
   SmallKPlan sk;
 };
 
-// Threads and vertices per thread of the register descent: the smallest block that covers n with 4
-// vertices per thread (measured on the plain configuration, n = 1000, k = 5: 256 x 4 beats 128 x 8 by 10%
-// and 512 x 4 by 50%); CCB_REG_SHAPE=T,V overrides it for tuning sweeps.
+// Threads and vertices per thread of the register descent.  Up to 1023 vertices (compact pairs, issue-bound: few warps,
+// whose per-move overhead is paid once each) the fewest warps that hold n at 4, then 8 vertices a thread; above, the
+// smallest block that covers n with 4.  CCB_REG_SHAPE=T,V overrides it for tuning sweeps.
 void RegisterShape(int n, int* threads, int* vpt) {
   *vpt = 4;
-  *threads = 128;
-  while (*threads * *vpt < n) *threads *= 2;
+  if (n <= 256) {
+    *threads = 64;
+  } else if (n <= 512) {
+    *threads = 128;
+  } else if (n <= 1023) {
+    *threads = 128;
+    *vpt = 8;
+  } else {
+    *threads = 512;
+    while (*threads * *vpt < n) *threads *= 2;
+  }
   if (const char* env = std::getenv("CCB_REG_SHAPE")) {
     int t = 0, v = 0;
     if (std::sscanf(env, "%d,%d", &t, &v) == 2 && RegistersShapeBuilt(t, v) && t * v >= n) {
@@ -511,7 +520,8 @@ struct ccb_solver {
   int32_t* cur_sizes = nullptr;
   int64_t* cur_f = nullptr;
   int64_t* next_f = nullptr;
-  uint32_t* masks = nullptr;
+  uint32_t* masks = nullptr;   // popcount rebuild: cluster masks (allocated when it is used)
+  uint8_t* z = nullptr;        // tensor rebuild: one-hot labels (likewise)
   int64_t* intra = nullptr;    // tiled rebuild (wide path): per-slot intra-cluster sums; null: per-slot rebuild
   int rebuild_kind = CCB_REBUILD_AUTO;
   bool plain = true;  // iterated by the plain path's kernels (false: by the batched engine's, which rebuild by popcount)
@@ -626,26 +636,31 @@ void SetRebuild(ccb_solver& s, int kind) {
                           "with n >= 128");
   }
   s.rebuild_kind = kind;
-  if (!WantTensor(s, kind)) {
-    s.tensor.reset();
-    return;
+  std::unique_ptr<TensorRebuild> t;
+  if (WantTensor(s, kind)) {
+    if (s.tensor) return;
+    t.reset(new TensorRebuild());
+    const char* why = nullptr;
+    PlanTensorRebuild(*t, s.n, s.pop * s.k, s.device.sms, &why);
+    const size_t z_bytes = (size_t)t->z_rows * t->kz;
+    if (!s.plan.wide && s.z == nullptr) {  // by popcount where Z would take memory the caller may count on
+      size_t free_b = 0, total_b = 0;
+      CCB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      if (z_bytes > free_b / 4) t.reset();
+    }
+    if (t) {
+      if (s.z == nullptr) {
+        s.Alloc(s.z, z_bytes);
+        const size_t live = (size_t)s.pop * s.k * t->kz;  // written whole by every rebuild; the rows past it stay zero
+        if (z_bytes > live) CCB_CUDA(cudaMemset(s.z + live, 0, z_bytes - live));
+        s.device_bytes += z_bytes;
+      }
+      if (s.intra == nullptr) s.Alloc(s.intra, s.pop);
+      CCB_CUDA(EncodeTensorRebuild(*t, s.graph->bits, s.graph->pitch, s.z));
+    }
   }
-  if (s.tensor) return;
-  std::unique_ptr<TensorRebuild> t(new TensorRebuild());
-  const char* why = nullptr;
-  PlanTensorRebuild(*t, s.n, s.pop * s.k, s.device.sms, &why);
-  if (!s.plan.wide) {  // the popcount rebuild where Z would take memory the caller may count on
-    size_t free_b = 0, total_b = 0;
-    CCB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if ((size_t)t->z_rows * t->kz > free_b / 4) return;
-    if (s.intra == nullptr) s.Alloc(s.intra, s.pop);
-  }
-  uint8_t* z = nullptr;
-  s.Alloc(z, (size_t)t->z_rows * t->kz);
-  CCB_CUDA(cudaMemset(z, 0, (size_t)t->z_rows * t->kz));
-  CCB_CUDA(EncodeTensorRebuild(*t, s.graph->bits, s.graph->pitch, z));
-  s.device_bytes += (size_t)t->z_rows * t->kz;
   s.tensor = std::move(t);
+  if (!s.tensor && s.masks == nullptr) s.Alloc(s.masks, (size_t)s.pop * s.k * s.graph->pitch);
 }
 
 ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool plain = true) {
@@ -691,7 +706,6 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   s->Alloc(s->cur_sizes, (size_t)pop * s->kpad);
   s->Alloc(s->cur_f, pop);
   s->Alloc(s->next_f, pop);
-  s->Alloc(s->masks, (size_t)pop * k * g->pitch);
   // Wide graphs do not fit L2: rebuild G with each row read once for all slots (a tile of 16 rows per block in
   // shared memory) instead of once per slot.
   if (s->plan.wide && (size_t)kRebuildTileThreads / kWarp * g->pitch * 4 + 2048 <= (size_t)s->device.smem_optin) {
