@@ -3,91 +3,156 @@
 // run by the CLI at include/cc_cli.hpp:337-343) and of State::Rebuild (src/cc_pbils_cpu.cpp:74-95).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include "ccb.h"
 #include "ccb_device.cuh"
 #include "ccb_error.h"
+#include "ccb_util.h"
 
 namespace ccb {
 namespace {
 
-constexpr int kEvalThreads = 512;
-constexpr int kEvalChunk = 8;
+constexpr int kEvalThreads = 256;
+constexpr int kEvalWarps = kEvalThreads / kWarp;
 
-// One block per labeling.  Phase 1 packs a bit mask per cluster with warp ballots into `masks`
-// ([labeling][k][words], scratch) and counts cluster sizes; every mask word is written before it is
-// read, so the scratch needs no clearing.  Phase 2 gives each warp whole rows: lanes stride over the
-// row's words and count the bits shared with each cluster's mask, reduced across the warp in hardware.
-// A label outside [0, k) marks the labeling invalid: its f is written as -1.
+// Three launches per call, each over the whole chip whatever the count (one block per labeling left all but one SM idle
+// for the recount of a single solution: n = 20000, k = 16 took 15 ms, now about 0.1):
+//   k_eval_masks   one bit mask per cluster by warp ballots into `masks` ([labeling][k][words], scratch), f zeroed;
+//   k_eval_rows    G = popc(row & mask), a warp per kRows rows and kChunk clusters, so that a mask word loaded serves
+//                  kRows rows; each block adds its rows' own-cluster counts to f;
+//   k_eval_finish  sizes from the masks, f = edges + sum_c C(size_c, 2) - (the sum so far).  A label outside [0, k) is
+//                  in no mask: the sizes then sum to less than n and f is -1.
+// Bound by POPC (8 clocks a warp): n k ceil(n / 32) of them per labeling.
 __global__ void __launch_bounds__(kEvalThreads)
-    k_evaluate(const uint32_t* __restrict__ bits, int n, int words, int pitch, long long edges, int k,
-               const int32_t* __restrict__ all_labels, uint32_t* __restrict__ masks, int64_t* __restrict__ f_out,
-               int32_t* __restrict__ sizes_out, int32_t* __restrict__ g_out) {
-  constexpr int kWarps = kEvalThreads / kWarp;
-  __shared__ int s_sizes[kMaxK];
-  __shared__ int s_bad;
-  __shared__ long long s_sum[kWarps];
+    k_eval_masks(const int32_t* __restrict__ all_labels, int n, int words, int k, uint32_t* __restrict__ masks,
+                 int64_t* __restrict__ f_out) {
   const int sol = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int lane = tid % kWarp;
-  const int warp = tid / kWarp;
+  const int lane = threadIdx.x % kWarp;
   const int32_t* labels = all_labels + static_cast<size_t>(sol) * n;
   uint32_t* my_masks = masks + static_cast<size_t>(sol) * k * words;
-  for (int c = tid; c < k; c += kEvalThreads) s_sizes[c] = 0;
-  if (tid == 0) s_bad = 0;
-  __syncthreads();
-
-  for (int w = warp; w < words; w += kWarps) {
+  if (blockIdx.y == 0 && threadIdx.x == 0) f_out[sol] = 0;
+  for (int w = blockIdx.y * kEvalWarps + threadIdx.x / kWarp; w < words; w += gridDim.y * kEvalWarps) {
     const int v = w * kWarp + lane;
     const int l = v < n ? labels[v] : -1;
-    if (v < n && (l < 0 || l >= k)) s_bad = 1;
     for (int c = 0; c < k; ++c) {
       const uint32_t m = __ballot_sync(kAllLanes, l == c);
-      if (lane == (c % kWarp)) {
-        my_masks[static_cast<size_t>(c) * words + w] = m;
-        if (m) atomicAdd(&s_sizes[c], __popc(m));
-      }
+      if (lane == (c % kWarp)) my_masks[static_cast<size_t>(c) * words + w] = m;
     }
   }
-  __syncthreads();
+}
 
-  long long intra_twice = 0;
-  for (int v = warp; v < n; v += kWarps) {
-    const uint32_t* row = bits + static_cast<size_t>(v) * pitch;
-    const int own = labels[v];
-    for (int c0 = 0; c0 < k; c0 += kEvalChunk) {
-      int acc[kEvalChunk];
+template <int kChunk, int kRows>
+__global__ void __launch_bounds__(kEvalThreads)
+    k_eval_rows(const uint32_t* __restrict__ bits, int n, int words, int pitch, int k,
+                const int32_t* __restrict__ all_labels, const uint32_t* __restrict__ masks, int64_t* __restrict__ f_out,
+                int32_t* __restrict__ g_out) {
+  __shared__ long long s_sum[kEvalWarps];
+  const int sol = blockIdx.x;
+  const int lane = threadIdx.x % kWarp;
+  const int v0 = (blockIdx.y * kEvalWarps + threadIdx.x / kWarp) * kRows;
+  const int32_t* labels = all_labels + static_cast<size_t>(sol) * n;
+  const uint32_t* my_masks = masks + static_cast<size_t>(sol) * k * words;
+  long long own_sum = 0;
+  if (v0 < n) {
+    const int rows = min(kRows, n - v0);
+    const int own = lane < rows ? labels[v0 + lane] : -1;
+    for (int c0 = 0; c0 < k; c0 += kChunk) {
+      int acc[kRows][kChunk];
 #pragma unroll
-      for (int i = 0; i < kEvalChunk; ++i) acc[i] = 0;
+      for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) acc[r][i] = 0;
+      }
       for (int w = lane; w < words; w += kWarp) {
-        const uint32_t a = __ldg(row + w);
+        uint32_t m[kChunk];
 #pragma unroll
-        for (int i = 0; i < kEvalChunk; ++i)
-          if (c0 + i < k) acc[i] += __popc(a & my_masks[static_cast<size_t>(c0 + i) * words + w]);
+        for (int i = 0; i < kChunk; ++i) m[i] = c0 + i < k ? my_masks[static_cast<size_t>(c0 + i) * words + w] : 0u;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          const uint32_t a = r < rows ? __ldg(bits + static_cast<size_t>(v0 + r) * pitch + w) : 0u;
+#pragma unroll
+          for (int i = 0; i < kChunk; ++i) acc[r][i] += __popc(a & m[i]);
+        }
       }
 #pragma unroll
-      for (int i = 0; i < kEvalChunk; ++i) {
-        if (c0 + i < k) {
-          const int total = static_cast<int>(__reduce_add_sync(kAllLanes, static_cast<unsigned>(acc[i])));
-          if (lane == 0) {
-            if (g_out != nullptr) g_out[(static_cast<size_t>(sol) * k + c0 + i) * n + v] = total;
-            if (own == c0 + i) intra_twice += total;
-          }
+      for (int i = 0; i < kChunk; ++i) {
+        if (c0 + i >= k) break;
+        int mine = 0;  // lane r: row r's count
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          const int total = __reduce_add_sync(kAllLanes, acc[r][i]);
+          mine = lane == r ? total : mine;
+        }
+        if (lane < rows) {
+          if (g_out != nullptr) g_out[(static_cast<size_t>(sol) * k + c0 + i) * n + v0 + lane] = mine;
+          if (own == c0 + i) own_sum += mine;
         }
       }
     }
   }
-  const long long sum = BlockSum<kWarps>(intra_twice, s_sum);
-  if (tid == 0) {
-    long long pairs = 0;
-    for (int c = 0; c < k; ++c) pairs += static_cast<long long>(s_sizes[c]) * (s_sizes[c] - 1) / 2;
-    f_out[sol] = s_bad ? -1 : edges + pairs - sum;
+  const long long sum = BlockSum<kEvalWarps>(own_sum, s_sum);
+  if (threadIdx.x == 0 && sum != 0) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(f_out + sol), static_cast<unsigned long long>(sum));
   }
+}
+
+__global__ void __launch_bounds__(kEvalThreads)
+    k_eval_finish(const uint32_t* __restrict__ masks, int n, int words, int k, long long edges,
+                  int64_t* __restrict__ f_out, int32_t* __restrict__ sizes_out) {
+  __shared__ int s_sizes[kMaxK];
+  const int sol = blockIdx.x;
+  const int lane = threadIdx.x % kWarp;
+  const uint32_t* my_masks = masks + static_cast<size_t>(sol) * k * words;
+  for (int c = threadIdx.x / kWarp; c < k; c += kEvalWarps) {  // a warp per cluster
+    int size = 0;
+    for (int w = lane; w < words; w += kWarp) size += __popc(my_masks[static_cast<size_t>(c) * words + w]);
+    size = __reduce_add_sync(kAllLanes, size);
+    if (lane == 0) s_sizes[c] = size;
+  }
+  __syncthreads();
   if (sizes_out != nullptr) {
-    for (int c = tid; c < k; c += kEvalThreads) sizes_out[static_cast<size_t>(sol) * k + c] = s_sizes[c];
+    for (int c = threadIdx.x; c < k; c += kEvalThreads) sizes_out[static_cast<size_t>(sol) * k + c] = s_sizes[c];
   }
+  if (threadIdx.x == 0) {
+    long long pairs = 0, placed = 0;
+    for (int c = 0; c < k; ++c) {
+      pairs += static_cast<long long>(s_sizes[c]) * (s_sizes[c] - 1) / 2;
+      placed += s_sizes[c];
+    }
+    f_out[sol] = placed < n ? -1 : edges + pairs - f_out[sol];
+  }
+}
+
+template <int kChunk, int kRows>
+void LaunchEvalRows(const uint32_t* bits, int n, int words, int pitch, int k, int count, const int32_t* labels,
+                    const uint32_t* masks, int64_t* f_out, int32_t* g_out, cudaStream_t st) {
+  const dim3 grid(count, (n + kEvalWarps * kRows - 1) / (kEvalWarps * kRows));  // <= 32768 for n <= 2^20
+  k_eval_rows<kChunk, kRows><<<grid, kEvalThreads, 0, st>>>(bits, n, words, pitch, k, labels, masks, f_out, g_out);
+}
+
+cudaError_t LaunchEvaluate(const uint32_t* bits, int n, int pitch, uint64_t edges, int k, int count,
+                           const int32_t* labels, uint32_t* masks, int64_t* f_out, int32_t* sizes_out, int32_t* g_out,
+                           cudaStream_t st) {
+  const int words = (n + 31) / 32;
+  const int parts = std::max(1, std::min((words + kEvalWarps - 1) / kEvalWarps, (256 + count - 1) / count));
+  k_eval_masks<<<dim3(count, parts), kEvalThreads, 0, st>>>(labels, n, words, k, masks, f_out);
+  if (n > 0) {
+    // kChunk * kRows counters a thread: as many rows as the clusters leave
+    if (k <= 4) {
+      LaunchEvalRows<4, 16>(bits, n, words, pitch, k, count, labels, masks, f_out, g_out, st);
+    } else if (k <= 8) {
+      LaunchEvalRows<8, 8>(bits, n, words, pitch, k, count, labels, masks, f_out, g_out, st);
+    } else {
+      LaunchEvalRows<16, 4>(bits, n, words, pitch, k, count, labels, masks, f_out, g_out, st);
+    }
+  }
+  k_eval_finish<<<count, kEvalThreads, 0, st>>>(masks, n, words, k, (long long)edges, f_out, sizes_out);
+  return cudaGetLastError();
 }
 
 const char* CheckEvaluateArgs(const uint32_t* bits, uint32_t n, uint32_t words_per_row, int32_t k, int32_t count,
@@ -106,7 +171,65 @@ int Report(int status, const char* message) {
   return status;
 }
 
+// Whether a recount is faster as the tensor-core contraction (ccb_evaluate_labelings_tensor, the same integers), by what
+// both were measured to take (B200): popcount 4.2 M row-word intersections a us, the contraction 1.25 us a K step of 128
+// vertices and wave of CTAs (256 vertices x 256 columns each), 10 us more of set-up.  n = 20000, k = 16: 106 us against
+// 150 for one labeling, 4290 against 480 for 64; n = 4001, k = 64, 32 labelings: 455 against 83.
+bool PreferTensorRecount(const uint32_t* bits, int n, int words_per_row, int k, int count) {
+  if (n < 128 || words_per_row % 4 != 0 || reinterpret_cast<uintptr_t>(bits) % 16 != 0) return false;
+  const double words = (n + 31) / 32, columns = (double)count * k;
+  if (columns * words * 32 > 1024.0 * 1024 * 1024 || columns > 1 << 24) return false;  // its one-hot scratch
+  const double waves = std::ceil(std::ceil(n / 256.0) * std::ceil(columns / 256) / 148);
+  return 10 + waves * std::ceil(words / 4) * 1.25 < n * words * columns / 4.2e6;
+}
+
+constexpr int kScratchMaxDevices = 64;
+constexpr uint64_t kScratchKept = 64ull << 20;  // bytes a device's pool keeps between calls
+std::mutex g_scratch_mutex;
+cudaMemPool_t g_scratch_pool[kScratchMaxDevices] = {};
+
 }  // namespace
+
+// The default pool gives its memory back at every synchronisation, so each recount mapped its scratch anew (0.2 ms, up to
+// several on a busy host).  A pool of our own per device keeps up to kScratchKept; ccb_release_cache trims it.  Stream
+// ordered and thread safe like the default pool, which serves captures and devices without pool support.
+cudaError_t ScratchAlloc(void** out, size_t bytes, cudaStream_t st) {
+  int device = 0;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaMemPool_t pool = nullptr;
+  if (cudaGetDevice(&device) == cudaSuccess && device < kScratchMaxDevices &&
+      cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (g_scratch_pool[device] == nullptr) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.handleTypes = cudaMemHandleTypeNone;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      uint64_t kept = kScratchKept;
+      if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept) == cudaSuccess) {
+          g_scratch_pool[device] = pool;
+        } else {
+          cudaMemPoolDestroy(pool);
+        }
+      }
+    }
+    pool = g_scratch_pool[device];
+  }
+  if (pool != nullptr && cudaMallocFromPoolAsync(out, bytes, pool, st) == cudaSuccess) return cudaSuccess;
+  cudaGetLastError();  // what failed above is tried again below
+  return cudaMallocAsync(out, bytes, st);
+}
+
+void ScratchTrim() {
+  std::lock_guard<std::mutex> lock(g_scratch_mutex);
+  for (cudaMemPool_t pool : g_scratch_pool) {
+    if (pool != nullptr) cudaMemPoolTrimTo(pool, 0);
+  }
+  cudaGetLastError();
+}
+
 }  // namespace ccb
 
 using namespace ccb;
@@ -120,18 +243,22 @@ int ccb_evaluate_labelings(const uint32_t* bits, uint32_t n, uint32_t words_per_
     return Report(CCB_ERR_INVALID, why);
   }
   if (count == 0) return Report(CCB_OK, "");
+  if (PreferTensorRecount(bits, (int)n, (int)words_per_row, k, count)) {
+    const int status = ccb_evaluate_labelings_tensor(bits, n, words_per_row, edges, k, count, labels, f_out, sizes_out,
+                                                     g_out, stream);
+    if (status != CCB_ERR_DEVICE_MEMORY) return status;  // else by popcount, with a tenth of the scratch
+    cudaGetLastError();
+  }
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int words = (int)((n + 31) / 32);
   const size_t mask_bytes = sizeof(uint32_t) * (size_t)count * k * words;
   uint32_t* masks = nullptr;
   cudaError_t e = cudaSuccess;
   if (mask_bytes > 0) {
-    e = cudaMallocAsync(&masks, mask_bytes, st);
+    e = ScratchAlloc(reinterpret_cast<void**>(&masks), mask_bytes, st);
     if (e != cudaSuccess) return Report(CCB_ERR_DEVICE_MEMORY, cudaGetErrorString(e));
   }
-  k_evaluate<<<count, kEvalThreads, 0, st>>>(bits, (int)n, words, (int)words_per_row, (long long)edges, k, labels,
-                                             masks, f_out, sizes_out, g_out);
-  e = cudaGetLastError();
+  e = LaunchEvaluate(bits, (int)n, (int)words_per_row, edges, k, count, labels, masks, f_out, sizes_out, g_out, st);
   if (masks) cudaFreeAsync(masks, st);
   if (e != cudaSuccess) return Report(CCB_ERR_CUDA, cudaGetErrorString(e));
   return Report(CCB_OK, "");
@@ -146,7 +273,7 @@ int ccb_evaluate_labelings(const uint32_t* bits, uint32_t n, uint32_t words_per_
 // memory is already reserved by its own pool allocator (a framework that took the free memory up
 // front, where cudaMalloc fails or fragments that pool), or a latency-critical loop that must not pay
 // cudaMalloc / cudaFree, which can synchronise the whole device.  For them the mask scratch of
-// k_evaluate lives in a fixed array in device memory, loaded with the library: every GPU that loads
+// the recount lives in a fixed array in device memory, loaded with the library: every GPU that loads
 // libccb.so holds these kNoAllocMaskWords words (4 MiB) until the process exits.
 //
 // The array's host-side name is only a stand-in, not a device address, so the entry point looks the
@@ -158,13 +285,11 @@ int ccb_evaluate_labelings(const uint32_t* bits, uint32_t n, uint32_t words_per_
 // CUDA_MODULE_LOADING=EAGER the array is allocated when the library is loaded.)  The address is kept for
 // the life of the process: after cudaDeviceReset on a device the module is loaded afresh and may sit
 // elsewhere, so the entry point must not be used across a device reset.
-// Every call shares the one array and finds the last call's contents there.  k_evaluate writes every
+// Every call shares the one array and finds the last call's contents there.  The recount writes every
 // mask word it later reads, so nothing needs clearing between calls; but two calls whose kernels
 // overlap on the GPU (different streams, or different host threads) race on the array, so callers
 // must order their calls.
 // ------------------------------------------------------------------------------------------------
-#include <mutex>
-
 namespace ccb {
 namespace {
 
@@ -214,9 +339,8 @@ int ccb_evaluate_labelings_noalloc(const uint32_t* bits, uint32_t n, uint32_t wo
   cudaError_t e = NoAllocScratch(&masks);  // also the whole of a count = 0 call: the per-device set-up
   if (e != cudaSuccess) return Report(CCB_ERR_CUDA, cudaGetErrorString(e));
   if (count == 0) return Report(CCB_OK, "");
-  k_evaluate<<<count, kEvalThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      bits, (int)n, (int)words, (int)words_per_row, (long long)edges, k, labels, masks, f_out, sizes_out, g_out);
-  e = cudaGetLastError();
+  e = LaunchEvaluate(bits, (int)n, (int)words_per_row, edges, k, count, labels, masks, f_out, sizes_out, g_out,
+                     static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return Report(CCB_ERR_CUDA, cudaGetErrorString(e));
   return Report(CCB_OK, "");
 }

@@ -10,6 +10,7 @@
 
 #include "ccb.h"
 #include "ccb_error.h"
+#include "ccb_util.h"
 
 namespace ccb {
 namespace {
@@ -663,7 +664,7 @@ int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t wor
   const size_t sizes_bytes = sizes_out ? 0 : (size_t)count * kpad * 4;
   const size_t scratch = z_bytes + (size_t)count * 8 + (size_t)count * 4 + 16 + sizes_bytes;
   uint8_t* buf = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void**>(&buf), scratch, st);
+  e = ScratchAlloc(reinterpret_cast<void**>(&buf), scratch, st);
   if (e != cudaSuccess) return report(CCB_ERR_DEVICE_MEMORY, cudaGetErrorString(e));
   uint8_t* z = buf;
   int64_t* intra = reinterpret_cast<int64_t*>(buf + z_bytes);  // z_bytes is a multiple of 128

@@ -2366,7 +2366,10 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
 
 }  // namespace
 
-void ccb_release_cache(void) { t_cache.Release(); }
+void ccb_release_cache(void) {
+  t_cache.Release();
+  ScratchTrim();
+}
 
 int ccb_pbils_solve(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges,
                     const ccb_params* params, int32_t* labels_out, ccb_result* result) {

@@ -37,6 +37,11 @@ struct Failure {
     }                                                                                                      \
   } while (0)
 
+// Scratch of a recount from the library's own stream-ordered pool (freed with cudaFreeAsync), and its return to the
+// device (ccb_evaluate.cu).
+cudaError_t ScratchAlloc(void** out, size_t bytes, cudaStream_t st);
+void ScratchTrim();
+
 [[noreturn]] inline void Fail(int status, const std::string& message) { throw Failure{status, message}; }
 
 template <typename F>

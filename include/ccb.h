@@ -92,7 +92,8 @@ int ccb_neighborhood_solve(const uint32_t* bits, uint32_t n, uint32_t words_per_
  * (graph rows, population, scratch) and reuse them when the next call on the same device has the same n, k,
  * population and ls_kernel: a repeated solve then pays the bitset upload, not the allocations.  No
  * counterpart in the reference, whose calls allocate and free everything (cuda/cc_pbils_gpu.cu:105-122).
- * ccb_release_cache frees the calling thread's buffers; they are also freed when the thread exits. */
+ * ccb_release_cache frees the calling thread's buffers; they are also freed when the thread exits.  It also gives
+ * back the recounts' scratch memory (at most 64 MiB per device is kept between calls). */
 void ccb_release_cache(void);
 
 /* ---- device-resident graphs and reusable solvers ----------------------------------------------
@@ -261,8 +262,9 @@ void ccb_server_destroy(ccb_server* server);
  * called from include/cc_cli.hpp:337-343) and of State::Rebuild (src/cc_pbils_cpu.cpp:74-95).
  * Device pointers: bits (n rows of words_per_row words), labels [count][n] int32, f_out [count];
  * sizes_out [count][k] and g_out [count][k][n] (int32, cluster-major) may be NULL.  A labeling with a
- * label outside [0, k) gets f = -1.  Scratch (count * k * ceil(n/32) mask words) is taken from the
- * stream-ordered allocator for the call.  Asynchronous on `stream`. */
+ * label outside [0, k) gets f = -1.  Scratch (count * k * ceil(n/32) mask words) is taken from a
+ * stream-ordered pool for the call.  Large batches over 16-byte aligned rows run as the contraction of
+ * ccb_evaluate_labelings_tensor (the same outputs).  Asynchronous on `stream`. */
 int ccb_evaluate_labelings(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k,
                            int32_t count, const int32_t* labels, int64_t* f_out, int32_t* sizes_out,
                            int32_t* g_out, void* stream);
