@@ -38,7 +38,7 @@ struct BatchShape {
   bool window = false;  // the windowed descent in the place of the kind's own kernel
   int k = 0;            // compile-time K of the register, streamed and windowed (k <= 8) forms
   int threads = 256;
-  int vpt = 4;          // register forms; windowed: members per scan thread
+  int vpt = 4;          // register forms
   bool smem = false;    // register form: bitset in shared memory; streamed / incremental: state in shared memory
   size_t smem_bytes = 0;
   int blocks_per_sm = 0;  // tuned resident slots per SM (0: the occupancy limit)

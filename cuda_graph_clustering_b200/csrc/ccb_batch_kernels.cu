@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kWindowThreads, 1) kb_descent_window(const Bat
   __shared__ int s_item;
   int entry, slot;
   while (ClaimItem(q, &s_item, entry, slot)) {
-    DescentWindow<K, S, int16_t>(CurrentDescent(entries[entry]), slot);
+    DescentWindow<K, kWindowCap, S, int16_t>(CurrentDescent(entries[entry]), slot);
     __syncthreads();
   }
 }
@@ -286,7 +286,7 @@ template <int K, bool S>
 __global__ void __launch_bounds__(kWindowThreads, 1) kf_window(const BatchEntry* __restrict__ entries, FlowState* flow,
                                                                FlowBucket b) {
   FlowLoop<kWindowThreads>(entries, flow, b, [](const DescentArgs<int16_t>& a, int slot) {
-    DescentWindow<K, S, int16_t>(a, slot);
+    DescentWindow<K, kWindowCap, S, int16_t>(a, slot);
   });
 }
 

@@ -42,19 +42,21 @@ namespace ccb {
 constexpr int kWindowMoves = 64;   // most moves of a window (two 32-bit vectors)
 constexpr int kWindowBins = 128;   // gains above the lower bound that a threshold can take
 constexpr int kWindowThreads = 512;
-constexpr int kWindowCap = 1024;         // most members of a window
+constexpr int kWindowCap = 1024;         // most members of a window (k <= 8 also runs with more)
 constexpr int kWindowPenalty = 1 << 26;  // own-cluster bias of a member's keys (2^20 in units of h)
 constexpr int kWindowAbsent = 1 << 25;   // key of a cluster past k: above every foreign key, below every own one
 
 // How the members' moves are made for a cluster bound: with all K keys of a member in registers (`keys` of them, k
 // padded to it), or (keys = 0) with its counters in shared memory and its best key cached; and by how many threads,
-// each with Members() of them.
+// for at most `cap` members.
 struct WindowForm {
   int keys, threads;
-  __host__ __device__ constexpr int Members() const { return kWindowCap / threads; }
 };
-__host__ __device__ constexpr WindowForm WindowFormOf(int k) {
-  return k <= 8 ? WindowForm{k, 256} : k <= 16 ? WindowForm{16, 256} : k <= 32 ? WindowForm{32, 512} : WindowForm{0, 512};
+__host__ __device__ constexpr WindowForm WindowFormOf(int k, int cap) {
+  return k <= 8    ? WindowForm{k, cap > kWindowCap ? 512 : 256}
+         : k <= 16 ? WindowForm{16, 256}
+         : k <= 32 ? WindowForm{32, 512}
+                   : WindowForm{0, 512};
 }
 
 // The bound of a cluster count that an instance is compiled for: k itself up to 8, then 16, 32, 64.
@@ -107,12 +109,13 @@ __device__ __forceinline__ void WindowScanBarrier() {
 }
 
 // State of a block's windows in shared memory.
+template <int kCap>
 struct WindowShared {
   uint4 mask[kMaxK][2];      // per cluster and 32 moves: F | T, F, popc(F), (first entry) 64 size + c
   int off[kMaxK];            // 64 size_c + c
   int hist[kWindowBins];
   int warp_count[kWindowThreads / kWarp];
-  int member[kWindowCap];    // vertices of S, ascending
+  int member[kCap];          // vertices of S, ascending except at k <= 8
   int move_v[kWindowMoves];
   int move_ft[kWindowMoves];  // from | to << 8
   uint32_t record[2][kWindowThreads / kWarp];  // each scan warp's best move key
@@ -148,7 +151,8 @@ struct WindowBook {
     ++moves;
   }
   // The window's end, by one thread: `gain` is the best member's.
-  __device__ __forceinline__ void Close(WindowShared& s, int theta, int gain) const {
+  template <int kCap>
+  __device__ __forceinline__ void Close(WindowShared<kCap>& s, int theta, int gain) const {
     // with a move cap of 1 the vertices outside S may have the best gain itself
     const int bound = theta - (s.move_cap == 1 ? 1 : 0) - top1 - top2;
     s.moves = moves;
@@ -174,14 +178,17 @@ __device__ __forceinline__ void WithCluster(int c, F&& f) {
 
 // The moves of one window with a member's K keys 64 h_c + c in registers (k <= K clusters; the own key biased by
 // kWindowPenalty, so that the minimum of the keys is the best foreign target and the maximum the own cluster), V
-// members per thread.  Move keys are field << kField | member << 2 kC | from << kC | to with field = gain - L +
-// kBias, clamped.  Leaves in s the moves, the new lower bound and whether no vertex can improve.
-template <int K, int V, int T>
+// members per thread.  Move keys are field << kField | id << 2 kC | from << kC | to with field = gain - L + kBias,
+// clamped, and id the vertex (K <= 8, n <= 65536: the row address comes from the key itself) or the member.  Leaves in s the moves, the new lower bound and whether no vertex can improve.
+template <int K, int V, int T, int kCap>
 __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const uint16_t* g, int ldw, uint8_t* lab,
-                                             WindowShared& s, long long& objective) {
+                                             WindowShared<kCap>& s, long long& objective) {
   constexpr int kC = K <= 8 ? 3 : 5;  // bits of a cluster in a move key
-  constexpr int kField = 2 * kC + 11;
-  constexpr uint32_t kFieldMax = (1u << (31 - kField)) - 1u;
+  constexpr bool kByVertex = K <= 8;
+  constexpr int kIdBits = kByVertex ? 16 : 11;
+  constexpr uint32_t kIdMask = ((1u << kIdBits) - 1u) << (2 * kC);
+  constexpr int kField = 2 * kC + kIdBits;
+  constexpr uint32_t kFieldMax = (1u << ((kByVertex ? 32 : 31) - kField)) - 1u;
   constexpr int kBias = 256;
   constexpr int kClusterMask = (1 << kC) - 1;
   constexpr int kWarps = T / kWarp;
@@ -200,7 +207,7 @@ __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const u
     const int i = j * T + tid;
     const bool ok = i < count;
     su[j] = s.member[ok ? i : 0];
-    code[j] = ok ? static_cast<uint32_t>(i) << (2 * kC) : ~0u;
+    code[j] = ok ? static_cast<uint32_t>(kByVertex ? su[j] : i) << (2 * kC) : ~0u;
     const int own = lab[su[j]];
     const uint16_t* gu = g + WindowPlace(su[j]);
 #pragma unroll
@@ -270,8 +277,8 @@ __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const u
     const int gain = static_cast<int>(best >> kField) - kBias + low;
     // below theta - D the best member is the best vertex; a gain of 0 or more is no move
     if (book.moves >= cap || gain >= min(theta - book.top1 - book.top2, 0) || (best >> kField) >= kFieldMax) break;
-    const int moved = static_cast<int>((best >> (2 * kC)) & 2047u);
-    const int v = s.member[moved];
+    const int id = static_cast<int>((best & kIdMask) >> (2 * kC));
+    const int v = kByVertex ? id : s.member[id];
     const uint32_t* row = gr.bits + static_cast<size_t>(v) * gr.pitch;
 #pragma unroll
     for (int j = 0; j < V; ++j) rw[j] = row[su[j] >> 5];
@@ -282,7 +289,13 @@ __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const u
       for (int c = 0; c < K; ++c) coef[c] = (c == from ? 1 : 0) - (c == to ? 1 : 0);
     }
     objective += gain;
-    mine = moved % T == tid ? moved / T : -1;
+    if constexpr (kByVertex) {
+      mine = -1;
+#pragma unroll
+      for (int j = 0; j < V; ++j) mine = code[j] == (best & kIdMask) ? j : mine;
+    } else {
+      mine = id % T == tid ? id / T : -1;
+    }
     if (mine >= 0) {
       lab[v] = static_cast<uint8_t>(to);
       s.move_v[book.moves] = v;
@@ -383,7 +396,7 @@ __device__ __forceinline__ int2 WindowRescan(const uint16_t* g, int ld, int i, i
 // gain - L + 128, clamped; to = from marks a bound.
 template <int V, int T, int kCap>
 __device__ __forceinline__ void WindowMovesN(const GraphView& gr, int k, const WindowMembers<kCap>& mem, uint8_t* lab,
-                                             WindowShared& s, long long& objective) {
+                                             WindowShared<kCap>& s, long long& objective) {
   constexpr uint32_t kFieldMax = 511u;
   constexpr int kBias = 128;
   constexpr int kWarps = T / kWarp;
@@ -513,16 +526,15 @@ __device__ __forceinline__ void WindowMovesN(const GraphView& gr, int k, const W
 // One slot's descent.  K: the cluster count at compile time (2 .. 8), or the bound of a runtime one (16, 32, 64) that
 // picks how the moves are made.  kSmemG: the counters in shared memory, else
 // in the slot's rows of `next` (leading dimension WindowLd(n) either way).  GainT: the population's G.
-template <int kBound, bool kSmemG, typename GainT>
+template <int kBound, int kCap, bool kSmemG, typename GainT>
 __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int slot) {
   constexpr int K = kBound <= 8 ? kBound : 0;
   constexpr int T = kWindowThreads;
   constexpr int kWarps = T / kWarp;
-  constexpr WindowForm kForm = WindowFormOf(kBound);
-  constexpr int V = kForm.Members();
-  constexpr int kCap = kWindowCap;
+  constexpr WindowForm kForm = WindowFormOf(kBound, kCap);
+  constexpr int V = kCap / kForm.threads;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ WindowShared s;
+  __shared__ WindowShared<kCap> s;
 
   const int tid = threadIdx.x;
   const int lane = tid % kWarp;
@@ -748,7 +760,7 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
       }
     }
     __syncthreads();
-    // ---- S in vertex order: each warp counts, then writes, the members of its own quads
+    // ---- S: each warp counts, then writes, the members of its own quads
     {
       const int bins = s.bins;
       auto members_of = [&](int quad) {  // bit t: vertex 32 t + lane of the quad is a member
@@ -761,13 +773,32 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
         const uint32_t in = members_of(quad);
         mine += (in & 1u) + ((in >> 1) & 1u) + ((in >> 2) & 1u) + (in >> 3);
       }
+      const uint32_t lane_members = mine;
       mine = __reduce_add_sync(kAllLanes, mine);
       if (lane == 0) s.warp_count[warp] = static_cast<int>(mine);
       __syncthreads();
       const int wc = lane < kWarps ? s.warp_count[lane] : 0;
       int at = __reduce_add_sync(kAllLanes, lane < warp ? wc : 0);
       const int total = __reduce_add_sync(kAllLanes, wc);
-      if (mine > 0) {
+      if (kBound <= 8 && s.move_cap > 1) {
+        // move keys carry the vertex: any order will do, so a lane writes its own vertices one after another (no
+        // population counts, which take eight clocks each)
+        int incl = static_cast<int>(lane_members);
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+          const int y = __shfl_up_sync(kAllLanes, incl, o);
+          if (lane >= o) incl += y;
+        }
+        int p = at + incl - static_cast<int>(lane_members);
+        const int end = at + incl;
+        for (int quad = quad0; quad < quad1 && __any_sync(kAllLanes, p < end); ++quad) {
+          const uint32_t in = members_of(quad);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            if ((in >> t) & 1u) s.member[p++] = 128 * quad + 32 * t + lane;
+          }
+        }
+      } else if (mine > 0) {  // in vertex order: the lowest kCap of them where S cannot hold all
         const unsigned below = (1u << lane) - 1u;
         for (int quad = quad0; quad < quad1; ++quad) {
           const uint32_t in = members_of(quad);
@@ -791,7 +822,7 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
     __syncthreads();
     // ---- moves
     if constexpr (kForm.keys > 0) {
-      if (tid < kForm.threads) WindowMovesK<kForm.keys, V, kForm.threads>(a.gr, k, g, ldw, lab, s, objective);
+      if (tid < kForm.threads) WindowMovesK<kForm.keys, V, kForm.threads, kCap>(a.gr, k, g, ldw, lab, s, objective);
     } else {
       members.template Fill<T>(g, ldw, lab, s.member, s.members, s.off, k);
       __syncthreads();
@@ -812,9 +843,9 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
 }
 
 // One slot per block (plain path).
-template <int kBound, bool kSmemG, typename GainT>
+template <int kBound, int kCap, bool kSmemG, typename GainT>
 __global__ void __launch_bounds__(kWindowThreads, 1) k_descent_window(DescentArgs<GainT> a) {
-  DescentWindow<kBound, kSmemG, GainT>(a, blockIdx.x);
+  DescentWindow<kBound, kCap, kSmemG, GainT>(a, blockIdx.x);
 }
 
 }  // namespace ccb

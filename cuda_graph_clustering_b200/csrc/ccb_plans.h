@@ -19,7 +19,7 @@ struct SmallKPlan {
   bool smem_rows = false;   // whole bitset in shared memory
   size_t smem_bytes = 0;
   int cluster = 0;          // streamed form whose state does not fit one CTA: CTAs of the cluster holding it
-  bool window = false;      // the windowed descent (ccb_descent_window.cuh): vpt members per scan thread
+  bool window = false;      // the windowed descent (ccb_descent_window.cuh); k is its compiled bound
   bool l2_hints = false;    // streamed form from global memory: state loads/stores evict_last, rows evict_first
 };
 // The smallest cluster (2, 4 or 8 CTAs) whose shares of the packed state fit `limit` bytes of shared memory per
@@ -54,10 +54,12 @@ size_t Wide2Smem16Bytes(int n);
 size_t Wide3Smem26Bytes(int n);
 // Windowed descent: sets the plan's window fields for (n, k) within `limit` bytes of shared memory per block, returns
 // whether it fits; bytes of a slot's rows of `next` when the counters are not in shared memory.
-bool PlanWindow(SmallKPlan& plan, int n, int k, size_t limit);
+bool PlanWindow(SmallKPlan& plan, int n, int k, bool wide, size_t limit);
 size_t WindowGlobalBytes(int n, int k);
 cudaError_t LaunchDescentWindow(const SmallKPlan& plan, const DescentArgs<int16_t>& args, int grid,
                                 cudaStream_t stream, bool configure);
+cudaError_t LaunchDescentWindowWide(const SmallKPlan& plan, const DescentArgs<int32_t>& args, int grid,
+                                    cudaStream_t stream, bool configure);
 cudaError_t LaunchDescentSmallK(const SmallKPlan& plan, const DescentArgs<int16_t>& args, int grid,
                                 cudaStream_t stream, bool configure);
 

@@ -252,6 +252,18 @@ bool PreferWindow(int n, int k, int64_t edges, bool rows_in_smem) {
   return n <= 1024 || (n <= 2200.0 * width && (k <= 32 || width >= 4.0));
 }
 
+// The same for the wide path (32767 < n <= 65536), whose windows hold up to 4096 members at k <= 4.  us a move (B200, the
+// kernel without windows -> windowed; vertices per unit of gain width in brackets):
+//   k = 2, whose degree-proportional kernel is cheap: G(50001, 0.1) [376] 5.4 -> 2.2, but G(33000, 0.02) [656] 2.2 -> 2.4;
+//   k = 3: G(65536, 0.02) [1130] 8.3 -> 4.2, but G(65536, 0.005) [2250] 4.5 -> 6.2;
+//   k >= 4: G(40000, 0.05), k = 6 [800] 35 -> 3.3; G(40000, 0.01), k = 8 [2030] 39 -> 8.0; G(65536, 0.01), k = 9 [2750]
+//     59 -> 23.
+bool PreferWindowWide(int n, int k, int64_t edges) {
+  const double p = 2.0 * (double)edges / ((double)n * (n - 1));
+  const double width = 2.8 * std::sqrt(std::max(0.0, n * p * (1.0 - p) / k));
+  return n <= (k == 2 ? 500.0 : k == 3 ? 1500.0 : 4000.0) * width;
+}
+
 // Bytes of the population's descent scratch in global memory (the slots' rows of `next`); 0 when the state is in
 // shared memory or registers.
 size_t NextBytes(const Plan& plan, int n, int k, int ld, int pop) {
@@ -337,7 +349,7 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
   }
   if (!p.wide && k >= 2 && ls_kernel == CCB_LS_AUTO && PreferWindow(n, k, edges, p.small_k && p.sk.smem_rows)) {
     SmallKPlan w;
-    if (PlanWindow(w, n, k, limit)) {
+    if (PlanWindow(w, n, k, false, limit)) {
       p.sk = w;
       p.small_k = k <= 8;
       p.incremental = k > 8;
@@ -345,6 +357,18 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
       p.smem_rows = false;
       p.threads = w.threads;
       p.smem_bytes = w.smem_bytes;
+    }
+  }
+  if (p.wide && n <= kMaxVerticesIncrementalWide && k >= 2 && ls_kernel == CCB_LS_AUTO && PreferWindowWide(n, k, edges)) {
+    // uint16 counters: exact while every degree < 65536
+    SmallKPlan w;
+    if (PlanWindow(w, n, k, true, limit)) {
+      p.sk = w;
+      p.smem_state = false;
+      p.smem_rows = false;
+      p.threads = w.threads;
+      p.smem_bytes = w.smem_bytes;
+      return p;
     }
   }
   if (p.wide && (k == 2 || k == 3) && ls_kernel == CCB_LS_AUTO) {
@@ -412,6 +436,7 @@ void LaunchDescent(const Plan& p, const DescentArgs<GainT>& a, int grid, cudaStr
 }
 
 const char* KernelName(const Plan& p) {
+  if (p.wide && p.sk.window) return "windowed wide (n <= 65536, uint16 counters), counters in L2";
   if (p.packed_wide) {
     if (p.sk.k == 3) {
       if (p.smem16) return "packed wide k = 3, degree-proportional (per-thread best of each (cluster, target) class), "
@@ -725,7 +750,9 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   CCB_CUDA(cudaEventCreateWithFlags(&s->poll_event[1], cudaEventDisableTiming));
 
   // Shared-memory opt-in for the descent instance of this plan.
-  if ((s->plan.incremental && s->plan.wide) || s->plan.packed_wide) {
+  if (s->plan.wide && s->plan.sk.window) {
+    CCB_CUDA(LaunchDescentWindowWide(s->plan.sk, DescentArgs<int32_t>{}, 0, nullptr, true));
+  } else if ((s->plan.incremental && s->plan.wide) || s->plan.packed_wide) {
     // no dynamic shared memory
   } else if (s->plan.sk.window) {
     CCB_CUDA(LaunchDescentWindow(s->plan.sk, DescentArgs<int16_t>{}, 0, nullptr, true));
@@ -830,6 +857,12 @@ void LaunchDescentStep(ccb_solver& s, int grid, int population, int tournament, 
       return;
     }
   } else {
+    if (s.plan.sk.window) {
+      cudaError_t e = cudaSuccess;
+      s.timer.Time(kCatDescent, st, [&] { e = LaunchDescentWindowWide(s.plan.sk, a, grid, st, false); });
+      CCB_CUDA(e);
+      return;
+    }
     if (s.plan.packed_wide) {
       cudaError_t e = cudaSuccess;
       s.timer.Time(kCatDescent, st, [&] { e = LaunchDescentWidePacked(a, grid, s.plan.sparse, s.plan.smem16, st); });

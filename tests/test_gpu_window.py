@@ -56,3 +56,19 @@ def test_one_call_cache_follows_the_density(ccb, oracle, cuda_device):
     assert _plan(ccb, *dense, **p).startswith("windowed") and not _plan(ccb, *empty, **p).startswith("windowed")
     for bits, edges in (dense, empty, dense):
         _solve(ccb, oracle, bits, edges, **p)
+
+
+# The wide form (32767 < n <= 65536, int32 population) against the generic wide kernel on the same graph: first and
+# ragged sizes, the member caps of k <= 4, k <= 8 and larger k, every way the moves are made
+@pytest.mark.parametrize("n,k,density", [(32768, 4, 0.02), (32897, 3, 0.05), (33003, 2, 0.3), (32769, 7, 0.05),
+                                         (32800, 9, 0.05), (32770, 20, 0.1), (32900, 40, 0.2)])
+def test_wide_matches_the_generic_kernel(ccb, cuda_device, n, k, density):
+    graph = ccb.DeviceGraph.erdos_renyi(n, density, n + k)
+    p = dict(k=k, population=3, iterations=1, early_stop=10, seed=n)
+    auto = ccb.Solver(graph, ccb.PbilsParams(**p))
+    assert auto.describe().startswith("windowed wide")
+    got = auto.pbils(ccb.PbilsParams(**p))
+    want = ccb.Solver(graph, ccb.PbilsParams(**p, ls_kernel=ccb.LS_WIDE)).pbils(
+        ccb.PbilsParams(**p, ls_kernel=ccb.LS_WIDE))
+    assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+    assert np.array_equal(got.labels, want.labels)
