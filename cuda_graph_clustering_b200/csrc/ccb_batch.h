@@ -36,6 +36,7 @@ enum BatchKind : int { kBatchRegisters = 0, kBatchStream = 1, kBatchIncremental 
 struct BatchShape {
   int kind = kBatchRegisters;
   bool window = false;  // the windowed descent in the place of the kind's own kernel
+  bool half = false;    // its 16-bit form
   int k = 0;            // compile-time K of the register, streamed and windowed (k <= 8) forms
   int threads = 256;
   int vpt = 4;          // register forms

@@ -60,13 +60,13 @@ __global__ void __launch_bounds__(T, 1) kb_descent_stream(const BatchEntry* __re
   }
 }
 
-template <int K, bool S>
+template <int K, bool S, bool kHalf>
 __global__ void __launch_bounds__(kWindowThreads, 1) kb_descent_window(const BatchEntry* __restrict__ entries,
                                                                        BatchQueue q) {
   __shared__ int s_item;
   int entry, slot;
   while (ClaimItem(q, &s_item, entry, slot)) {
-    DescentWindow<K, kWindowCap, S, int16_t>(CurrentDescent(entries[entry]), slot);
+    DescentWindow<K, kWindowCap, S, kHalf, int16_t>(CurrentDescent(entries[entry]), slot);
     __syncthreads();
   }
 }
@@ -282,11 +282,11 @@ __global__ void __launch_bounds__(T, 1) kf_stream(const BatchEntry* __restrict__
   FlowLoop<T>(entries, flow, b, [](const DescentArgs<int16_t>& a, int slot) { DescentStream<K, T, S>(a, slot); });
 }
 
-template <int K, bool S>
+template <int K, bool S, bool kHalf>
 __global__ void __launch_bounds__(kWindowThreads, 1) kf_window(const BatchEntry* __restrict__ entries, FlowState* flow,
                                                                FlowBucket b) {
   FlowLoop<kWindowThreads>(entries, flow, b, [](const DescentArgs<int16_t>& a, int slot) {
-    DescentWindow<K, kWindowCap, S, int16_t>(a, slot);
+    DescentWindow<K, kWindowCap, S, kHalf, int16_t>(a, slot);
   });
 }
 
@@ -344,8 +344,9 @@ cudaError_t WithKernel(const BatchShape& s, F&& f) {
   if constexpr (kFlow) { return f(KF); } else { return f(KB); }
 #define CCB_WINDOW(K)                                                                                   \
   if (s.window && s.k == K) {                                                                           \
-    if (s.smem) { CCB_PICK((kb_descent_window<K, true>), (kf_window<K, true>)) }                        \
-    CCB_PICK((kb_descent_window<K, false>), (kf_window<K, false>))                                      \
+    if (!s.half) { CCB_PICK((kb_descent_window<K, false, false>), (kf_window<K, false, false>)) }       \
+    if (s.smem) { CCB_PICK((kb_descent_window<K, true, true>), (kf_window<K, true, true>)) }            \
+    CCB_PICK((kb_descent_window<K, false, true>), (kf_window<K, false, true>))                          \
   }
   CCB_WINDOW(2) CCB_WINDOW(3) CCB_WINDOW(4) CCB_WINDOW(5) CCB_WINDOW(6) CCB_WINDOW(7) CCB_WINDOW(8)
   CCB_WINDOW(16) CCB_WINDOW(32) CCB_WINDOW(64)

@@ -7,9 +7,9 @@
 namespace ccb {
 namespace {
 
-template <int K, int kCap, bool S, typename GainT>
+template <int K, int kCap, bool S, bool kHalf, typename GainT>
 cudaError_t Go(const SmallKPlan& p, const DescentArgs<GainT>& a, int grid, cudaStream_t st, bool configure) {
-  auto kernel = k_descent_window<K, kCap, S, GainT>;
+  auto kernel = k_descent_window<K, kCap, S, kHalf, GainT>;
   if (configure) return RaiseDynamicSmem(kernel, p.smem_bytes);
   if (grid > 0) kernel<<<grid, kWindowThreads, p.smem_bytes, st>>>(a);
   return cudaGetLastError();
@@ -17,8 +17,9 @@ cudaError_t Go(const SmallKPlan& p, const DescentArgs<GainT>& a, int grid, cudaS
 
 template <int kBound>
 cudaError_t ByPlacement(const SmallKPlan& p, const DescentArgs<int16_t>& a, int grid, cudaStream_t st, bool cfg) {
-  return p.smem_state ? Go<kBound, kWindowCap, true>(p, a, grid, st, cfg)
-                      : Go<kBound, kWindowCap, false>(p, a, grid, st, cfg);
+  if (!p.half) return Go<kBound, kWindowCap, false, false>(p, a, grid, st, cfg);
+  return p.smem_state ? Go<kBound, kWindowCap, true, true>(p, a, grid, st, cfg)
+                      : Go<kBound, kWindowCap, false, true>(p, a, grid, st, cfg);
 }
 
 // Members of the wide form's windows: as many as their keys leave registers for, since a refresh passes over twice the
@@ -27,7 +28,7 @@ constexpr int WideCap(int k) { return k <= 4 ? 4 * kWindowCap : k <= 8 ? 2 * kWi
 
 template <int kBound>
 cudaError_t Wide(const SmallKPlan& p, const DescentArgs<int32_t>& a, int grid, cudaStream_t st, bool cfg) {
-  return Go<kBound, WideCap(kBound), false>(p, a, grid, st, cfg);
+  return Go<kBound, WideCap(kBound), false, false>(p, a, grid, st, cfg);
 }
 
 }  // namespace
@@ -42,7 +43,8 @@ bool PlanWindow(SmallKPlan& p, int n, int k, bool wide, size_t limit) {
   const size_t fixed = 8 * 1024 + (size_t)cap * 4;  // the kernels' static shared memory
   if (limit < fixed) return false;
   limit -= fixed;
-  p.smem_state = !wide && WindowSmem(n, k, true, cap) <= limit;
+  p.half = n <= kWindowHalfMax;
+  p.smem_state = p.half && WindowSmem(n, k, true, cap) <= limit;
   p.smem_bytes = WindowSmem(n, k, p.smem_state, cap);
   return p.smem_bytes <= limit;
 }

@@ -18,6 +18,10 @@
 // (WarpTranspose32).  With F and T the masks of the moves leaving and entering c, the counter changes by
 // popc(x & T) - popc(x & F) = popc((x ^ F) & (F | T)) - popc(F).
 //
+// Up to n = 16383 (kHalf) the slot's array holds h_c(u) itself in 16 bits, biased by 2^14, with the top bit set in u's own
+// cluster: a pair of vertices then takes one multiply-add to update, one 16-bit pair minimum (the best foreign h) and one
+// maximum (the own) per cluster, and no label is read.  Above, where h needs 17 bits, it holds the counters G_c(u).
+//
 // If more than kWindowCap vertices share the best gain, the members are the kWindowCap lowest of them and the window
 // ends after one move (the lowest such vertex is the best move; nothing is known after it).
 //
@@ -39,6 +43,7 @@
 
 namespace ccb {
 
+constexpr int kWindowHalfMax = 16383;  // largest n whose h fit 15 bits
 constexpr int kWindowMoves = 64;   // most moves of a window (two 32-bit vectors)
 constexpr int kWindowBins = 128;   // gains above the lower bound that a threshold can take
 constexpr int kWindowThreads = 512;
@@ -180,7 +185,7 @@ __device__ __forceinline__ void WithCluster(int c, F&& f) {
 // kWindowPenalty, so that the minimum of the keys is the best foreign target and the maximum the own cluster), V
 // members per thread.  Move keys are field << kField | id << 2 kC | from << kC | to with field = gain - L + kBias,
 // clamped, and id the vertex (K <= 8, n <= 65536: the row address comes from the key itself) or the member.  Leaves in s the moves, the new lower bound and whether no vertex can improve.
-template <int K, int V, int T, int kCap>
+template <int K, int V, int T, int kCap, bool kHalf>
 __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const uint16_t* g, int ldw, uint8_t* lab,
                                              WindowShared<kCap>& s, long long& objective) {
   constexpr int kC = K <= 8 ? 3 : 5;  // bits of a cluster in a move key
@@ -208,11 +213,14 @@ __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const u
     const bool ok = i < count;
     su[j] = s.member[ok ? i : 0];
     code[j] = ok ? static_cast<uint32_t>(kByVertex ? su[j] : i) << (2 * kC) : ~0u;
-    const int own = lab[su[j]];
+    const int own = kHalf ? 0 : lab[su[j]];
     const uint16_t* gu = g + WindowPlace(su[j]);
 #pragma unroll
     for (int c = 0; c < K; ++c) {
-      if (K <= 8 || c < k) {
+      if (kHalf && (K <= 8 || c < k)) {  // h + 2^14 in every key: the gains are the same
+        const int x = gu[static_cast<size_t>(c) * ldw];
+        key[j][c] = 64 * (x & 0x7fff) + c + (x >= 0x8000 ? kWindowPenalty : 0);
+      } else if (K <= 8 || c < k) {
         key[j][c] = s.off[c] - 128 * static_cast<int>(gu[static_cast<size_t>(c) * ldw]) + (c == own ? kWindowPenalty : 0);
       } else {
         key[j][c] = kWindowAbsent;
@@ -321,7 +329,7 @@ struct WindowMembers {
     own = bound + kCap;
   }
   // All threads: the members' counters from g, their keys with them.
-  template <int kThreads>
+  template <int kThreads, bool kHalf>
   __device__ __forceinline__ void Fill(const uint16_t* counters, int ldw, const uint8_t* lab, const int* member,
                                        int count, const int* off, int k) {
     for (int i = threadIdx.x; i < count; i += kThreads) {
@@ -331,10 +339,11 @@ struct WindowMembers {
       int b1 = 0x7fffffff, b2 = 0x7fffffff, ko = 0;
 #pragma unroll 16
       for (int c = 0; c < k; ++c) {
-        const uint16_t x = counters[static_cast<size_t>(c) * ldw + at];
-        g[c * kLd + i] = x;
+        int x = counters[static_cast<size_t>(c) * ldw + at];
         const int offc = off[c];
-        const int key = offc - 128 * static_cast<int>(x);
+        if constexpr (kHalf) x = ((offc >> 6) - (x & 0x7fff) + 0x4000) >> 1;  // G = (size - h) / 2
+        g[c * kLd + i] = static_cast<uint16_t>(x);
+        const int key = offc - 128 * x;
         if (c == o) {
           ko = key;
         } else if (offc >= 64) {
@@ -524,9 +533,9 @@ __device__ __forceinline__ void WindowMovesN(const GraphView& gr, int k, const W
 }
 
 // One slot's descent.  K: the cluster count at compile time (2 .. 8), or the bound of a runtime one (16, 32, 64) that
-// picks how the moves are made.  kSmemG: the counters in shared memory, else
+// picks how the moves are made.  kHalf: n <= 16383 (see above).  kSmemG: the counters in shared memory, else
 // in the slot's rows of `next` (leading dimension WindowLd(n) either way).  GainT: the population's G.
-template <int kBound, int kCap, bool kSmemG, typename GainT>
+template <int kBound, int kCap, bool kSmemG, bool kHalf, typename GainT>
 __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int slot) {
   constexpr int K = kBound <= 8 ? kBound : 0;
   constexpr int T = kWindowThreads;
@@ -571,6 +580,8 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
   if constexpr (kForm.keys == 0) members.Carve(smem + static_cast<size_t>(ldw) * 2 * (1 + (kSmemG ? k : 0)), k);
   {
     const GainT* g_src = a.cur.g + static_cast<size_t>(w) * k * ld;
+    const uint8_t* lab_src = a.cur.labels + static_cast<size_t>(w) * ld;
+    const int32_t* sizes = a.cur.sizes + static_cast<size_t>(w) * a.kpad;
     for (int i = warp; i < k * quads; i += kWarps) {
       const int c = i / quads, quad = i - c * quads;
       uint32_t x[4];
@@ -578,14 +589,17 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
       for (int t = 0; t < 4; ++t) {
         const int u = 128 * quad + 32 * t + lane;
         x[t] = u < ld ? static_cast<uint16_t>(g_src[static_cast<size_t>(c) * ld + u]) : 0u;
+        if constexpr (kHalf) {  // places past n are never read back
+          const uint32_t own = u < n && lab_src[u] == c ? 0x8000u : 0u;
+          x[t] = u < n ? static_cast<uint32_t>(sizes[c] - 2 * static_cast<int>(x[t]) + 0x4000) | own : 0x4000u;
+        }
       }
       reinterpret_cast<uint2*>(g + static_cast<size_t>(c) * ldw)[32 * quad + lane] =
           make_uint2(x[0] | x[1] << 16, x[2] | x[3] << 16);
     }
-    const uint4* ls = reinterpret_cast<const uint4*>(a.cur.labels + static_cast<size_t>(w) * ld);
+    const uint4* ls = reinterpret_cast<const uint4*>(lab_src);
     uint4* ldst = reinterpret_cast<uint4*>(lab);
     for (int i = tid; i < ld / 16; i += T) ldst[i] = ls[i];
-    const int32_t* sizes = a.cur.sizes + static_cast<size_t>(w) * a.kpad;
     for (int c = tid; c < k; c += T) s.off[c] = 64 * sizes[c] + c;
   }
   long long objective = a.cur.f[w];
@@ -607,11 +621,21 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
       const uint32_t f0 = __ballot_sync(kAllLanes, (ft0 & 0xff) == c), t0 = __ballot_sync(kAllLanes, (ft0 >> 8) == c);
       const uint32_t f1 = __ballot_sync(kAllLanes, (ft1 & 0xff) == c), t1 = __ballot_sync(kAllLanes, (ft1 >> 8) == c);
       if (lane == 0) {
-        const int off = s.off[c] + 64 * (__popc(t0) + __popc(t1) - __popc(f0) - __popc(f1));
+        const int left = __popc(f0) + __popc(f1), grown = __popc(t0) + __popc(t1) - left;
+        const int off = s.off[c] + 64 * grown;
         s.off[c] = off;
-        s.mask[c][0] = make_uint4(f0 | t0, f0, __popc(f0), static_cast<uint32_t>(off));
+        // kHalf: h changes by grown + 2 left - 2 popc((x ^ F) & (F | T)), of a pair at once
+        s.mask[c][0] = make_uint4(f0 | t0, f0, kHalf ? static_cast<uint32_t>(grown + 2 * left) * 0x10001u : __popc(f0),
+                                  static_cast<uint32_t>(off));
         s.mask[c][1] = make_uint4(f1 | t1, f1, __popc(f1), 0u);
       }
+    }
+    if (kHalf && tid < moves) {  // the moved vertices' own-cluster bits (flips: their order does not matter)
+      const int place = WindowPlace(s.move_v[tid]);
+      const uint32_t bit = 0x8000u << (16 * (place & 1));
+      uint32_t* words = reinterpret_cast<uint32_t*>(g) + place / 2;
+      atomicXor(words + static_cast<size_t>(s.move_ft[tid] & 0xff) * (ldw / 2), bit);
+      atomicXor(words + static_cast<size_t>(s.move_ft[tid] >> 8) * (ldw / 2), bit);
     }
     for (int b = tid; b < kWindowBins; b += T) s.hist[b] = 0;
     __syncthreads();
@@ -631,7 +655,7 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const int u = 128 * quad + 32 * t + lane;
-          next_own[t] = u < n ? lab[u] : 0;
+          next_own[t] = !kHalf && u < n ? lab[u] : 0;
         }
       };
       if (quad0 < quad1) read_ahead(quad0);
@@ -658,6 +682,7 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
         const size_t step = static_cast<size_t>(ldw) / 4;
         constexpr int kGroup = K > 0 ? K : 8;  // clusters whose loads are in flight together
         uint32_t left[4] = {0u, 0u, 0u, 0u};   // compile-time K: minus the changes so far (all changes sum to zero)
+        uint2 low2 = make_uint2(~0u, ~0u), high2 = make_uint2(0u, 0u);  // kHalf: smallest and largest h, in pairs
         for (int c0 = 0; c0 < k; c0 += kGroup) {
           uint2 gv[kGroup];
 #pragma unroll
@@ -670,41 +695,69 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
             if (K == 0 && c >= k) break;
             const uint4 m0 = s.mask[c][0];
             if (K > 0 ? moves > 0 : m0.x != 0u || (moves > kWarp && s.mask[c][1].x != 0u)) {
+              const bool last = K > 0 && i == K - 1;
               uint32_t d[4];
-              if (K > 0 && i == K - 1) {
+              if (!last) {
 #pragma unroll
-                for (int t = 0; t < 4; ++t) d[t] = left[t];
-              } else {
-#pragma unroll
-                for (int t = 0; t < 4; ++t) d[t] = __popc((x0[t] ^ m0.y) & m0.x) - m0.z;
+                for (int t = 0; t < 4; ++t) d[t] = __popc((x0[t] ^ m0.y) & m0.x);
                 if (moves > kWarp) {
                   const uint4 m1 = s.mask[c][1];
 #pragma unroll
-                  for (int t = 0; t < 4; ++t) d[t] += __popc((x1[t] ^ m1.y) & m1.x) - m1.z;
+                  for (int t = 0; t < 4; ++t) d[t] += __popc((x1[t] ^ m1.y) & m1.x) - (kHalf ? 0u : m1.z);
                 }
+              }
+              if constexpr (kHalf) {
+                uint32_t e0 = left[0], e1 = left[1];
+                if (!last) {
+                  e0 = m0.z - 2u * (d[0] + (d[1] << 16));
+                  e1 = m0.z - 2u * (d[2] + (d[3] << 16));
+                  left[0] -= e0;
+                  left[1] -= e1;
+                }
+                gv[i].x += e0;
+                gv[i].y += e1;
+              } else {
+#pragma unroll
+                for (int t = 0; t < 4; ++t) d[t] = last ? left[t] : d[t] - m0.z;
 #pragma unroll
                 for (int t = 0; t < 4; ++t) left[t] -= d[t];
+                gv[i].x += d[0] + (d[1] << 16);
+                gv[i].y += d[2] + (d[3] << 16);
               }
-              gv[i].x += d[0] + (d[1] << 16);
-              gv[i].y += d[2] + (d[3] << 16);
               gq[c * step] = gv[i];
             }
-            const int off = static_cast<int>(m0.w);
-            const int key[4] = {off - 128 * static_cast<int>(gv[i].x & 0xffffu), off - 128 * static_cast<int>(gv[i].x >> 16),
-                                off - 128 * static_cast<int>(gv[i].y & 0xffffu), off - 128 * static_cast<int>(gv[i].y >> 16)};
+            if constexpr (kHalf) {
+              low2.x = __vminu2(low2.x, gv[i].x);
+              low2.y = __vminu2(low2.y, gv[i].y);
+              high2.x = __vmaxu2(high2.x, gv[i].x);
+              high2.y = __vmaxu2(high2.y, gv[i].y);
+            } else {
+              const int off = static_cast<int>(m0.w);
+              const int key[4] = {off - 128 * static_cast<int>(gv[i].x & 0xffffu), off - 128 * static_cast<int>(gv[i].x >> 16),
+                                  off - 128 * static_cast<int>(gv[i].y & 0xffffu), off - 128 * static_cast<int>(gv[i].y >> 16)};
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const bool is_own = own[t] == c;
-              ko[t] = is_own ? key[t] : ko[t];
-              kmin[t] = min(kmin[t], is_own ? 0x7fffffff : key[t]);
+              for (int t = 0; t < 4; ++t) {
+                const bool is_own = own[t] == c;
+                ko[t] = is_own ? key[t] : ko[t];
+                kmin[t] = min(kmin[t], is_own ? 0x7fffffff : key[t]);
+              }
             }
           }
+        }
+        int gains[4];
+        if constexpr (kHalf) {
+          gains[0] = static_cast<int>(low2.x & 0xffffu) - static_cast<int>(high2.x & 0xffffu) + 0x8001;
+          gains[1] = static_cast<int>(low2.x >> 16) - static_cast<int>(high2.x >> 16) + 0x8001;
+          gains[2] = static_cast<int>(low2.y & 0xffffu) - static_cast<int>(high2.y & 0xffffu) + 0x8001;
+          gains[3] = static_cast<int>(low2.y >> 16) - static_cast<int>(high2.y >> 16) + 0x8001;
+        } else {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) gains[t] = (kmin[t] >> 6) - (ko[t] >> 6) + 1;
         }
         uint32_t d16[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          int gain = (kmin[t] >> 6) - (ko[t] >> 6) + 1;
-          if (u0 + 32 * t >= n) gain = 0x3fffffff;
+          const int gain = u0 + 32 * t < n ? gains[t] : 0x3fffffff;
           smallest = min(smallest, gain);
           d16[t] = static_cast<uint32_t>(min(gain - low, 65535));
           if (known_low && d16[t] < kWindowBins) atomicAdd(&s.hist[d16[t]], 1);
@@ -822,9 +875,9 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
     __syncthreads();
     // ---- moves
     if constexpr (kForm.keys > 0) {
-      if (tid < kForm.threads) WindowMovesK<kForm.keys, V, kForm.threads, kCap>(a.gr, k, g, ldw, lab, s, objective);
+      if (tid < kForm.threads) WindowMovesK<kForm.keys, V, kForm.threads, kCap, kHalf>(a.gr, k, g, ldw, lab, s, objective);
     } else {
-      members.template Fill<T>(g, ldw, lab, s.member, s.members, s.off, k);
+      members.template Fill<T, kHalf>(g, ldw, lab, s.member, s.members, s.off, k);
       __syncthreads();
       if (tid < kForm.threads) WindowMovesN<V, kForm.threads, kCap>(a.gr, k, members, lab, s, objective);
     }
@@ -843,9 +896,9 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
 }
 
 // One slot per block (plain path).
-template <int kBound, int kCap, bool kSmemG, typename GainT>
+template <int kBound, int kCap, bool kSmemG, bool kHalf, typename GainT>
 __global__ void __launch_bounds__(kWindowThreads, 1) k_descent_window(DescentArgs<GainT> a) {
-  DescentWindow<kBound, kCap, kSmemG, GainT>(a, blockIdx.x);
+  DescentWindow<kBound, kCap, kSmemG, kHalf, GainT>(a, blockIdx.x);
 }
 
 }  // namespace ccb

@@ -20,6 +20,7 @@ struct SmallKPlan {
   size_t smem_bytes = 0;
   int cluster = 0;          // streamed form whose state does not fit one CTA: CTAs of the cluster holding it
   bool window = false;      // the windowed descent (ccb_descent_window.cuh); k is its compiled bound
+  bool half = false;        // its 16-bit form, n <= 16383
   bool l2_hints = false;    // streamed form from global memory: state loads/stores evict_last, rows evict_first
 };
 // The smallest cluster (2, 4 or 8 CTAs) whose shares of the packed state fit `limit` bytes of shared memory per

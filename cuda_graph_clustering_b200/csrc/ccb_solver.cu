@@ -1241,6 +1241,7 @@ BatchShape ShapeOfPlan(const ccb_solver& s) {
   sh.vpt = sk.vpt;
   if (sk.window) {  // under the kind its sizes have without it, so that tuning entries find it
     sh.window = true;
+    sh.half = sk.half;
     sh.kind = s.k <= 8 ? (s.n <= 4096 ? kBatchRegisters : kBatchStream)
                        : (s.n <= 16384 ? kBatchIncrementalRegs : kBatchIncremental);
     sh.k = sk.k;
@@ -1278,10 +1279,10 @@ void BuildWorkLists(WorkLists& w, const std::vector<const ccb_solver*>& solvers,
                     double l2_share) {
   w.ReleaseBuckets();
   const int count = (int)solvers.size();
-  std::map<std::tuple<int, int, int, int, int, int, int, int>, int> index;
+  std::map<std::tuple<int, int, int, int, int, int, int, int>, int> index;  // window and half share one field
   for (int e = 0; e < count; ++e) {
     const BatchShape sh = ShapeOf(*solvers[e]);
-    const auto key = std::make_tuple((int)sh.window, sh.kind, sh.k, sh.threads, sh.vpt, (int)sh.smem, sh.blocks_per_sm, sh.max_slots);
+    const auto key = std::make_tuple(2 * (int)sh.window + (int)sh.half, sh.kind, sh.k, sh.threads, sh.vpt, (int)sh.smem, sh.blocks_per_sm, sh.max_slots);
     auto it = index.find(key);
     if (it == index.end()) {
       it = index.emplace(key, (int)w.buckets.size()).first;

@@ -28,7 +28,8 @@ def _plan(ccb, bits, edges, **p):
 @pytest.mark.parametrize("n,k,density", [
     (1281, 2, 0.3), (1314, 8, 0.3), (1315, 2, 0.3), (1408, 3, 0.5), (1409, 4, 0.2), (1535, 5, 0.4), (1537, 6, 0.3), (2047, 7, 0.3), (2049, 8, 0.6),
     (33, 9, 0.5), (128, 16, 0.4), (127, 17, 0.4), (129, 32, 0.3), (300, 33, 0.3), (64, 64, 0.5), (1025, 9, 0.2),
-    (2500, 16, 0.3), (1100, 32, 0.4), (1300, 64, 0.5), (9000, 13, 0.1), (12000, 8, 0.05)])
+    (2500, 16, 0.3), (1100, 32, 0.4), (1300, 64, 0.5), (9000, 13, 0.1), (12000, 8, 0.05),
+    (16383, 3, 0.3), (16384, 2, 0.3)])  # the largest n whose h fit 15 bits, and the first past it
 def test_matches_oracle(ccb, oracle, cuda_device, n, k, density):
     bits, edges = oracle.erdos_renyi(n, density, n + k)
     p = dict(k=k, population=4, iterations=3 if n < 3000 else 1, early_stop=10, gww=0.25, seed=n)
