@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kBatchRebuildThreads) kb_rebuild(const BatchEn
   while (ClaimItem(q, &s_item, entry, slot)) {
     RebuildArgs<int16_t> a = entries[entry].rebuild;
     a.iteration = a.ctl->iter;
-    RebuildBody<int16_t, kBatchRebuildThreads>(a, slot);
+    RebuildBody<int16_t, kBatchRebuildThreads>(a, slot, RebuildSource(a, slot));
     __syncthreads();
   }
 }
@@ -227,7 +227,7 @@ __device__ __forceinline__ void FlowLoop(const BatchEntry* __restrict__ entries,
     } else {
       RebuildArgs<int16_t> a = E.rebuild;
       a.iteration = iteration;
-      RebuildBody<int16_t, T>(a, slot);
+      RebuildBody<int16_t, T>(a, slot, RebuildSource(a, slot));
     }
     __syncthreads();
     if (threadIdx.x == 0) {

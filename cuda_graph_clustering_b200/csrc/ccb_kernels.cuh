@@ -79,13 +79,18 @@ struct RebuildArgs {
   int64_t* intra = nullptr;  // tiled form: labels, masks and sizes only; intra[slot] zeroed for the tiles
 };
 
+// The slot whose labels slot `slot` of the next population starts from.
+template <typename GainT>
+__device__ __forceinline__ int RebuildSource(const RebuildArgs<GainT>& a, int slot) {
+  return (a.mode == kRebuildPerturb || a.mode == kRebuildCopy) && a.src_map != nullptr ? a.src_map[slot] : slot;
+}
+
 template <typename GainT, int kThreads>
-__device__ __forceinline__ void RebuildBody(const RebuildArgs<GainT>& a, int slot) {
+__device__ __forceinline__ void RebuildBody(const RebuildArgs<GainT>& a, int slot, int src) {
   const GraphView& gr = a.gr;
   const PopView<GainT>& cur = a.cur;
   // plain (coherent) loads: in the batched flow kernel these are written by other blocks of the same launch
   const uint8_t* next_labels = a.next_labels;
-  const int32_t* src_map = a.src_map;
   uint32_t* __restrict__ masks = a.masks;
   const int k = a.k, kpad = a.kpad, ld = a.ld, mode = a.mode;
   const uint64_t stream = a.stream;
@@ -107,7 +112,6 @@ __device__ __forceinline__ void RebuildBody(const RebuildArgs<GainT>& a, int slo
   uint8_t* labels = cur.labels + static_cast<size_t>(slot) * ld;
 
   if (mode == kRebuildPerturb || mode == kRebuildCopy) {
-    const int src = src_map != nullptr ? src_map[slot] : slot;
     const uint8_t* from = next_labels + static_cast<size_t>(src) * ld;
     for (int v = tid; v < n; v += kThreads) {
       int l = from[v];
@@ -194,7 +198,7 @@ __device__ __forceinline__ void RebuildBody(const RebuildArgs<GainT>& a, int slo
 
 template <typename GainT, int kThreads>
 __global__ void __launch_bounds__(kThreads) k_rebuild(RebuildArgs<GainT> a) {
-  RebuildBody<GainT, kThreads>(a, blockIdx.x);
+  RebuildBody<GainT, kThreads>(a, blockIdx.x, RebuildSource(a, blockIdx.x));
 }
 
 // G = A*Z for every slot with each adjacency row read from memory once per rebuild (the one-block-per-slot
@@ -560,6 +564,48 @@ __device__ __forceinline__ void RecordBody(const RecordArgs& a) {
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads) k_record(RecordArgs a) {
   RecordBody<kThreads>(a);
+}
+
+// Record and rebuild of an iteration in one launch, for populations of at most kFusedSlots: block 0 keeps the record
+// beside its own slot's rebuild, and every block finds its slot's GWW source itself (its rank by one vote over the
+// block; only the worst `copies` slots rank the others).  The record alone, one block between two launches that wait for
+// it, took 8 of the 41 us of an iteration at n = 200, pop 32.
+constexpr int kFusedSlots = 256;
+template <typename GainT, int kThreads>
+__global__ void __launch_bounds__(kThreads) k_record_rebuild(RebuildArgs<GainT> a, RecordArgs r) {
+  static_assert(kThreads >= kFusedSlots, "a thread per slot");
+  __shared__ long long s_f[kFusedSlots];
+  __shared__ int s_stop, s_src;
+  const int slot = blockIdx.x;
+  const int tid = threadIdx.x;
+  // one thread reads the flag: block 0 of this launch may be setting it
+  if (tid == 0) s_stop = *reinterpret_cast<volatile int32_t*>(&r.ctl->stop);
+  if (tid < r.count) s_f[tid] = r.f[tid];
+  __syncthreads();
+  if (s_stop) return;
+  const int copies = r.copies;
+  if (slot == 0) {
+    r.copies = 0;
+    RecordBody<kThreads>(r);
+  }
+  int src = slot;
+  if (copies > 0) {
+    const long long f = s_f[slot];
+    const int rank = __syncthreads_count(tid < r.count && (s_f[tid] < f || (s_f[tid] == f && tid < slot)));
+    const int mirror = r.count - 1 - rank;  // the worst slots take the labels of the best, in order
+    if (mirror < copies) {
+      if (tid < r.count) {
+        const long long mine = s_f[tid];
+        int below = 0;
+        for (int t = 0; t < r.count; ++t) below += (s_f[t] < mine) || (s_f[t] == mine && t < tid);
+        if (below == mirror) s_src = tid;
+      }
+      __syncthreads();
+      src = s_src;
+    }
+  }
+  a.ctl = nullptr;  // the stop flag was looked at above, by the whole block alike
+  RebuildBody<GainT, kThreads>(a, slot, src);
 }
 
 }  // namespace ccb

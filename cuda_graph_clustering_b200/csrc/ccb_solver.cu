@@ -184,7 +184,7 @@ void RegisterShape(int n, int* threads, int* vpt) {
     *threads = 128;
     *vpt = 8;
   } else {
-    *threads = 512;
+    *threads = 256;
     while (*threads * *vpt < n) *threads *= 2;
   }
   if (const char* env = std::getenv("CCB_REG_SHAPE")) {
@@ -928,6 +928,16 @@ void LaunchPlainIteration(ccb_solver& s, const ccb_params& p, RecordArgs r, int 
   const bool perturb = s.k >= 2 && p.perturbation > 0.0;
   LaunchDescentStep<GainT>(s, s.pop, s.pop, p.tournament, it, StreamSeed(p.seed, kSelectTag, 0), st);
   r.iteration = it;
+  if (!s.tensor && s.intra == nullptr && s.pop <= kFusedSlots) {
+    const RebuildArgs<GainT> a{s.graph->View(), s.Cur<GainT>(), s.next_lab, nullptr, s.masks, s.k, s.kpad, s.ld,
+                               perturb ? kRebuildPerturb : kRebuildCopy, StreamSeed(p.seed, kPerturbTag, 0), it,
+                               (float)p.perturbation, 0, s.ctl};
+    s.timer.Time(kCatRebuild, st, [&] {
+      k_record_rebuild<GainT, kRebuildThreads><<<s.pop, kRebuildThreads, 0, st>>>(a, r);
+    });
+    CCB_CUDA(cudaGetLastError());
+    return;
+  }
   LaunchRecord(s, r, st);
   LaunchRebuild<GainT>(s, s.pop, perturb ? kRebuildPerturb : kRebuildCopy, copies > 0 ? s.src_map : nullptr,
                        StreamSeed(p.seed, kPerturbTag, 0), it, (float)p.perturbation, 0, true, st);
