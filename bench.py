@@ -594,7 +594,7 @@ def run_neighborhood(args, rank, world, local):
         per_move = n * (2 * 2 + 1) + 4 * words + 8 * deg  # SURVEY 8(d) generic move bytes at k = 2, sG = 2
         modelled = moves_per_launch * per_move / (descent_ms * 1e-3) / 1e9
         peak, peak_kind = measured_peak_hbm()
-        # the register descent (k = 2, 1024 threads x 4 vertices): issue roofline with the instructions per move
+        # the windowed descent (k = 2): issue roofline with the instructions per move
         # of its own ncu summary (profiles/k_descent_neighborhood.txt), the modelled bytes beside
         inst_per_move = profiled_value("k_descent_neighborhood", "warp_inst_per_move_per_block")
         sm_hz = (clock_info.get("sm_mhz") or 1965.0) * 1e6
@@ -602,9 +602,9 @@ def run_neighborhood(args, rank, world, local):
         ach = (inst_per_move or 0.0) * moves_per_launch / (descent_ms * 1e-3) / 1e9
         nb_roofline = {"bound": "issue", "achieved": ach if inst_per_move else None, "peak": issue_peak,
                        "unit": "G warp-inst/s", "frac": ach / issue_peak if inst_per_move else None,
-                       "traffic": profiled_traffic("k_descent_neighborhood"), "kernel": "k_descent_registers",
+                       "traffic": profiled_traffic("k_descent_neighborhood"), "kernel": "k_descent_window",
                        "avg_launch_ms": descent_ms,
-                       "limiter": "instruction issue (72 % of active cycles, ALU pipe 82 % on the SMs in use); "
+                       "limiter": "integer issue and the row latency of the members' moves; "
                                   "instructions per move from "
                                   "profiles/k_descent_neighborhood.txt",
                        "modelled_bytes": {"achieved_gbs": modelled, "hbm_peak_gbs": peak, "hbm_peak_kind": peak_kind,
@@ -820,10 +820,25 @@ def main():
             roofline = {"bound": "issue", "achieved": ach, "peak": issue_peak, "unit": "G warp-inst/s",
                         "frac": ach / issue_peak, "traffic": traffic, "kernel": "k_descent_registers",
                         "avg_launch_ms": descent_ms,
-                        "limiter": "latency of the per-move chain (row word, scan, warp minimum, block barrier); "
+                        "limiter": "integer issue (two clocks a warp instruction) of the per-move chain; "
                                    "instructions per move from profiles/k_descent_plain.txt",
                         "peak_kind": "issue slots of all SMs (4 per SM per cycle) at the sampled SM clock",
                         "modelled_bytes": modelled}
+        elif "windowed" in plan:
+            # a window scans a set of members per move and all vertices once per window: the modelled bytes per move
+            # are not what it moves, so its roofline is the instructions its ncu summary counted (null without one)
+            name = f"k_descent_window_{args.workload}"
+            inst_per_move = profiled_value(name, "warp_inst_per_move_per_block")
+            sm_hz = (clock_info.get("sm_mhz") or 1965.0) * 1e6
+            issue_peak = torch.cuda.get_device_properties(local).multi_processor_count * 4 * sm_hz / 1e9
+            ach = inst_per_move * moves_per_launch / (descent_ms * 1e-3) / 1e9 if inst_per_move else None
+            roofline = {"bound": "issue", "achieved": ach, "peak": issue_peak, "unit": "G warp-inst/s",
+                        "frac": ach / issue_peak if ach else None, "traffic": profiled_traffic(name),
+                        "kernel": "k_descent_window", "avg_launch_ms": descent_ms,
+                        "limiter": "integer issue of the members' moves and of the refresh, the latter with L2 "
+                                   f"bandwidth when its array is in L2; instructions per move from profiles/{name}.txt",
+                        "peak_kind": "issue slots of all SMs (4 per SM per cycle) at the sampled SM clock",
+                        "ns_per_move_per_slot": descent_ms * 1e6 / max(moves_per_launch / pop, 1.0)}
         elif "L2" in plan and l2_peak:
             roofline = {"bound": "l2", "achieved": achieved, "peak": l2_peak, "unit": "GB/s",
                         "frac": achieved / l2_peak, "traffic": traffic, "kernel": "k_descent",

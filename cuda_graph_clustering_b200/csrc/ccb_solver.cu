@@ -636,7 +636,8 @@ constexpr bool kTensorRebuildByDefault = true;
 // n = 1000, k = 5 (128K words a slot) 21 -> 32; n = 700, k = 16 (231K) 33 -> 32; n = 1000, k = 16 (480K) 46 -> 34; n =
 // 2000, k = 32 282 -> 65; n = 16000, k = 3 1902 -> 160; n = 32000, k = 8 13650 -> 988.
 bool PreferTensorNarrow(const ccb_solver& s) {
-  return s.n >= 128 && (long long)s.n * s.graph->words * (s.k - 1) >= 250000;
+  return s.n >= 128 && (long long)s.n * s.graph->words * (s.k - 1) >= 250000 &&
+         (long long)s.pop * s.k <= 1 << 22;  // column blocks within the grid's second dimension
 }
 
 // Whether the solver rebuilds G on the tensor cores: the tiled wide rebuild (int32 G) with n >= 128, chosen

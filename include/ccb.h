@@ -142,8 +142,9 @@ int ccb_solver_neighborhood(ccb_solver* solver, const ccb_params* params, int32_
  * popcount of cuda/cc_population_kernels.cuh:44-136 (KernelRebuild / KernelRebuild2).  CCB_REBUILD_TENSOR runs
  * the whole population's rebuild as one int8 contraction on the tensor cores (tcgen05 kind::i8, int32
  * accumulators in TMEM, operands fed by TMA): G[slot][c][v] = sum_u A[v][u] Z[slot*k + c][u] with Z the one-hot
- * labels.  The counts are the same integers either way, so every trajectory is unchanged.  It applies to the
- * wide path (int32 G: n > 32767, or ls_kernel CCB_LS_WIDE) with n >= 128; CCB_REBUILD_AUTO takes it there. */
+ * labels.  The counts are the same integers either way, so every trajectory is unchanged.  CCB_REBUILD_TENSOR applies
+ * to the wide path (int32 G: n > 32767, or ls_kernel CCB_LS_WIDE) with n >= 128; CCB_REBUILD_AUTO takes it there, and
+ * on the narrow path where the rebuild is large enough for it to be faster. */
 enum ccb_rebuild_kind { CCB_REBUILD_AUTO = 0, CCB_REBUILD_POPCOUNT = 1, CCB_REBUILD_TENSOR = 2 };
 int ccb_solver_set_rebuild(ccb_solver* solver, int32_t kind);
 /* Text description of the plan ("generic, shared memory, 512 threads, ..."). */
