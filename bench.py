@@ -835,8 +835,8 @@ def main():
             roofline = {"bound": "issue", "achieved": ach, "peak": issue_peak, "unit": "G warp-inst/s",
                         "frac": ach / issue_peak if ach else None, "traffic": profiled_traffic(name),
                         "kernel": "k_descent_window", "avg_launch_ms": descent_ms,
-                        "limiter": "integer issue of the members' moves and of the refresh, the latter with L2 "
-                                   f"bandwidth when its array is in L2; instructions per move from profiles/{name}.txt",
+                        "limiter": "integer issue of the members' moves and of the refresh, latency of rows and of "
+                                   f"an array in L2; instructions per move from profiles/{name}.txt",
                         "peak_kind": "issue slots of all SMs (4 per SM per cycle) at the sampled SM clock",
                         "ns_per_move_per_slot": descent_ms * 1e6 / max(moves_per_launch / pop, 1.0)}
         elif "L2" in plan and l2_peak:

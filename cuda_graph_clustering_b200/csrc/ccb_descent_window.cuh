@@ -25,14 +25,14 @@
 // If more than kWindowCap vertices share the best gain, the members are the kWindowCap lowest of them and the window
 // ends after one move (the lowest such vertex is the best move; nothing is known after it).
 //
-// What bounds it (B200, G(n, p), clocks per move of a slot at 1.965 GHz): the members' moves, about 850 at K = 3 and
-// 1090 at K = 8, are issue of 32-bit integer instructions (two warps per scheduler, two clocks each) plus 360 for the
+// What bounds it (B200, G(n, p), clocks per move of a slot at 1.965 GHz): the members' moves, about 835 at K = 3 and
+// 1060 at K = 8, are issue of 32-bit integer instructions (two warps per scheduler, two clocks each) plus 360 for the
 // row of the moved vertex from L2; four members on 256 threads measured best (K = 3: 2 x 512 threads 840 against 785,
 // 8 x 128 900; S of 512 or 2048 gives the refresh or the scan more than it takes from the other).  The refresh is one
-// pass over all vertices per window of 25 to 35 moves (n = 16000, k = 3: 16200 clocks, 570 a move; n = 32000, k = 8 with
-// its counters in L2: 61000, 2400 a move, L2 bandwidth), the choice of S 1800 to 7400.  A descent of 128 slots with one
-// scan of every vertex per move took, us per move: n = 16000, k = 3: 4.5, now 0.96; n = 32000, k = 8: 13.4, now 2.4;
-// n = 9001, k = 24: 11.9, now 2.9.
+// pass over all vertices per window of 25 to 35 moves: n = 16000, k = 3 505 a move (620 with counters, keys and labels
+// instead of h), n = 32000, k = 8 with its counters in L2 2280 (issue 54 %, L2 3.1 TB/s); the choice of S 75 to 270.  A
+// descent of 128 slots with one scan of every vertex per move took, us per move: n = 16000, k = 3: 4.5, now 0.85; n =
+// 32000, k = 8: 13.3, now 2.5; n = 9001, k = 24: 11.9, now 2.6.
 #pragma once
 
 #include <cstdint>
