@@ -248,6 +248,7 @@ __device__ __forceinline__ void DescentIncremental(const DescentArgs<GainT>& a, 
           chg |= static_cast<unsigned>(kb[i] != kb0 || ko[i] != ko0 || lbd[i] != lb0) << i;
           if (u == moved) st.lab[u] = static_cast<uint8_t>(to);
         }
+        __syncwarp();  // every lane's counters are visible to the warp's rescans
 #pragma unroll
         for (int i = 0; i < U; ++i) {
           unsigned m = __ballot_sync(kAllLanes, (need >> i) & 1u);
@@ -465,6 +466,7 @@ __device__ __forceinline__ void DescentIncrementalRegs(const DescentArgs<int16_t
             need |= 1u << i;
           }
         }
+        __syncwarp();  // every lane's counters are visible to the warp's rescans
         // warp-cooperative rescans, one vertex at a time
 #pragma unroll
         for (int i = 0; i < kGroup; ++i) {

@@ -468,6 +468,7 @@ __device__ __forceinline__ void WindowMovesN(const GraphView& gr, int k, const W
         }
         WindowFold(i == moved, offf - 128 * gf[j], offt - 128 * gt[j], from, to, from_empty, kb[j], lb[j], ko[j]);
       }
+      __syncwarp();  // every lane's counters are visible to the warp's rescans
     }
     best = ~0u;
 #pragma unroll

@@ -1,0 +1,37 @@
+"""Ordering that no result on one machine can show missing, looked for in the kernel sources (CPU only).
+
+A warp's rescans read counters that other lanes of the warp have just stored: votes and shuffles in between order no
+memory, so a __syncwarp() has to stand between the last store of a fold and the first vote that leads to a rescan.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cuda_graph_clustering_b200", "csrc")
+
+
+def source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+# file, function, the fold's last store of a counter, the rescan
+FOLDS = [
+    ("ccb_descent_window.cuh", "WindowMovesN", r"mem\.g\[to \* kLd \+ i\] =", r"WindowRescan\("),
+    ("ccb_descent_incremental.cuh", "DescentIncremental", r"st\.g\[static_cast<size_t>\(to\) \* ld \+ u\] =",
+     r"WarpRescan2\("),
+    ("ccb_descent_incremental.cuh", "DescentIncrementalRegs", r"\bg\[static_cast<size_t>\(to\) \* ld \+ u\] =",
+     r"WarpRescan2\("),
+]
+
+
+@pytest.mark.parametrize("name,function,store,rescan", FOLDS, ids=[f[1] for f in FOLDS])
+def test_warp_is_synchronised_between_the_fold_and_the_rescans(name, function, store, rescan):
+    text = source(name)
+    body = text[re.search(r"void " + function + r"\(", text).start():]
+    between = body[re.search(store, body).end():]
+    between = between[:re.search(rescan, between).start()]
+    vote = re.search(r"__ballot_sync\(", between)
+    assert vote is not None
+    assert "__syncwarp();" in between[:vote.start()]
