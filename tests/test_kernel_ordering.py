@@ -35,3 +35,11 @@ def test_warp_is_synchronised_between_the_fold_and_the_rescans(name, function, s
     vote = re.search(r"__ballot_sync\(", between)
     assert vote is not None
     assert "__syncwarp();" in between[:vote.start()]
+
+
+def test_tensor_memory_loads_wait_in_their_own_statement():
+    """A tcgen05.ld writes its registers after it was issued: the wait belongs to the same statement, so that nothing
+    that reads them can come in between."""
+    statements = re.findall(r"asm volatile\((.*?)\);", source("ccb_rebuild_tensor.cu"), flags=re.S)
+    loads = [s for s in statements if "tcgen05.ld." in s]
+    assert loads and all("tcgen05.wait::ld" in s for s in loads)
