@@ -22,8 +22,11 @@
 // cluster: a pair of vertices then takes one multiply-add to update, one 16-bit pair minimum (the best foreign h) and one
 // maximum (the own) per cluster, and no label is read.  Above, where h needs 17 bits, it holds the counters G_c(u).
 //
-// If more than kWindowCap vertices share the best gain, the members are the kWindowCap lowest of them and the window
-// ends after one move (the lowest such vertex is the best move; nothing is known after it).
+// If more than kWindowCap vertices share the best gain g, the members are the kWindowCap lowest of them and theta is g + 1.
+// The rest of them keep a gain of at least g - D = theta - 1 - D, and a member that reaches it is the lower vertex; every
+// other vertex stays at theta - D or above.  So the same test decides, and noise-free communities, whose vertices all tie
+// and whose gains fall by two with every move, get whole windows (with one move a window n = 16000, k = 3 took 8.3 us a
+// move, now 0.64; the kernel without windows 4.1).
 //
 // What bounds it (B200, G(n, p), clocks per move of a slot at 1.965 GHz): the members' moves, about 835 at K = 3 and
 // 1060 at K = 8, are issue of 32-bit integer instructions (two warps per scheduler, two clocks each) plus 360 for the
@@ -130,7 +133,7 @@ struct WindowShared {
   int smallest;   // smallest gain of the refresh
   int members;    // |S|
   int bins;       // theta - L
-  int move_cap;   // 1 when S holds only part of the vertices of the best gain
+  int partial;    // 1 when S holds only part of the vertices of the best gain
   int finished;
 };
 
@@ -158,8 +161,7 @@ struct WindowBook {
   // The window's end, by one thread: `gain` is the best member's.
   template <int kCap>
   __device__ __forceinline__ void Close(WindowShared<kCap>& s, int theta, int gain) const {
-    // with a move cap of 1 the vertices outside S may have the best gain itself
-    const int bound = theta - (s.move_cap == 1 ? 1 : 0) - top1 - top2;
+    const int bound = theta - s.partial - top1 - top2;  // partial: vertices outside S started at the best gain itself
     s.moves = moves;
     s.finished = gain >= 0 && bound >= 0;
     s.low = min(gain, bound);
@@ -203,7 +205,6 @@ __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const u
   const int count = s.members;
   const int low = s.low;
   const int theta = low + s.bins;
-  const int cap = s.move_cap;
   int key[V][K];
   int su[V];
   uint32_t code[V];
@@ -284,7 +285,7 @@ __device__ __forceinline__ void WindowMovesK(const GraphView& gr, int k, const u
     best = WarpMin(lane < kWarps ? rec[lane] : ~0u);
     const int gain = static_cast<int>(best >> kField) - kBias + low;
     // below theta - D the best member is the best vertex; a gain of 0 or more is no move
-    if (book.moves >= cap || gain >= min(theta - book.top1 - book.top2, 0) || (best >> kField) >= kFieldMax) break;
+    if (book.moves >= kWindowMoves || gain >= min(theta - book.top1 - book.top2, 0) || (best >> kField) >= kFieldMax) break;
     const int id = static_cast<int>((best & kIdMask) >> (2 * kC));
     const int v = kByVertex ? id : s.member[id];
     const uint32_t* row = gr.bits + static_cast<size_t>(v) * gr.pitch;
@@ -416,7 +417,6 @@ __device__ __forceinline__ void WindowMovesN(const GraphView& gr, int k, const W
   const int count = s.members;
   const int low = s.low;
   const int theta = low + s.bins;
-  const int cap = s.move_cap;
   // lane l: 64 size + c of clusters l and l + 32
   int off0 = lane < k ? s.off[lane] : 0x3fffffff;
   int off1 = lane + kWarp < k ? s.off[lane + kWarp] : 0x3fffffff;
@@ -505,7 +505,7 @@ __device__ __forceinline__ void WindowMovesN(const GraphView& gr, int k, const W
     WindowScanBarrier<T>();
     best = WarpMin(lane < kWarps ? rec[lane] : ~0u);
     const int gain = static_cast<int>(best >> 23) - kBias + low;
-    if (book.moves >= cap || gain >= min(theta - book.top1 - book.top2, 0) || (best >> 23) >= kFieldMax) break;
+    if (book.moves >= kWindowMoves || gain >= min(theta - book.top1 - book.top2, 0) || (best >> 23) >= kFieldMax) break;
     from = static_cast<int>((best >> 6) & 63u);
     to = static_cast<int>(best & 63u);
     near = (best & ~0x7fffffu) + (3u << 23);
@@ -809,7 +809,7 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
       bins = __reduce_max_sync(kAllLanes, bins);
       if (lane == 0) {
         const int least = smallest - s.low + 1;
-        s.move_cap = bins < least ? 1 : kWindowMoves;
+        s.partial = bins < least ? 1 : 0;
         s.bins = max(bins, least);
       }
     }
@@ -834,7 +834,7 @@ __device__ __forceinline__ void DescentWindow(const DescentArgs<GainT>& a, int s
       const int wc = lane < kWarps ? s.warp_count[lane] : 0;
       int at = __reduce_add_sync(kAllLanes, lane < warp ? wc : 0);
       const int total = __reduce_add_sync(kAllLanes, wc);
-      if (kBound <= 8 && s.move_cap > 1) {
+      if (kBound <= 8 && !s.partial) {
         // move keys carry the vertex: any order will do, so a lane writes its own vertices one after another (no
         // population counts, which take eight clocks each)
         int incl = static_cast<int>(lane_members);

@@ -1,0 +1,49 @@
+"""Which instances the windowed descent takes, and that it holds up where it could lose.
+
+Vertices whose gains tie by the thousand: a window of them makes as many moves as any other."""
+import numpy as np
+import pytest
+
+from oracle import make_params
+
+pytestmark = pytest.mark.gpu
+
+
+def _clock(ccb, solver, params):
+    """ns of descent a move, the better of three solves."""
+    solver.set_profiling(True)
+    best = None
+    for _ in range(3):
+        r = solver.pbils(params)
+        ns = solver.stats().descent_ms * 1e6 / max(r.accepted_moves, 1)
+        best = ns if best is None else min(best, ns)
+    return best
+
+
+# Two communities of more vertices than a window holds (1024), every gain of a community the same.  With one move a window
+# a move took 7.2 times as long as on the same communities with one pair in a thousand flipped, whose gains differ.
+@pytest.mark.parametrize("n,parts,k", [(6000, 2, 2), (5000, 2, 3)])
+def test_ties_cost_no_window_a_move(ccb, cuda_device, n, parts, k):
+    p = ccb.PbilsParams(k=k, population=64, iterations=2, early_stop=10, seed=3)
+    ns = []
+    for flip in (0.0, 0.001):
+        graph, _ = ccb.DeviceGraph.planted(n, parts, 1.0, 0.0, flip, 11)
+        solver = ccb.Solver(graph, p)
+        assert solver.describe().startswith("windowed")
+        ns.append(_clock(ccb, solver, p))
+    assert ns[0] < 4 * ns[1], ns
+
+
+# The same ties against the oracle: closed twins (gains fall together), open twins (they rise), classes of both, with windows
+# of vertex-keyed members (k <= 8), of members in order (k > 8) and of counters in shared memory (k > 32)
+@pytest.mark.parametrize("p_in,p_out", [(1.0, 0.0), (0.0, 1.0)])
+@pytest.mark.parametrize("n,parts,k", [(4000, 2, 3), (5000, 3, 4), (4100, 2, 16), (4200, 2, 40)])
+def test_ties_match_oracle(ccb, oracle, cuda_device, n, parts, k, p_in, p_out):
+    bits, edges, _ = oracle.planted(n, parts, False, p_in, p_out, 0.0, 5)
+    p = dict(k=k, population=2, iterations=2, early_stop=10, seed=2)
+    want = oracle.pbils(bits, edges, make_params(**p))
+    solver = ccb.Solver(ccb.DeviceGraph(ccb.Graph(n, bits, edges)), ccb.PbilsParams(**p))
+    assert solver.describe().startswith("windowed")
+    got = solver.pbils(ccb.PbilsParams(**p))
+    assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+    assert np.array_equal(got.labels, want.labels)
