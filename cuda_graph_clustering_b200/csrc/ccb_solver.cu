@@ -245,11 +245,27 @@ constexpr bool kClusterDescent = true;
 //   k > 8, at most 2200 a unit:  n = 9001, p = 0.2, k = 24 (230): 11.9 -> 2.9; n = 20000, p = 0.005, k = 9 (2140): 22.9
 //     -> 12.5; up to 1024 vertices all are members and no gain width is needed (n = 1000, p = 0.33, k = 16: 2.2 ->
 //     1.0).  With k > 32 and a width below 4 most keys tie: n = 4000, p = 0.02, k = 64 (width 3.1): 7.5 -> 9.7.
-bool PreferWindow(int n, int k, int64_t edges, bool rows_in_smem) {
+// An SM holds one windowed slot at a time, but two of the register descent at n <= 2048, k <= 5 and two to eight of the
+// incremental one at n <= 1024 (two while k n < 57000: its counters are in shared memory), so the line moves up once the
+// `slots` that run side by side fill the SMs more than once.  us a pass, without windows -> windowed:
+//   k <= 5, n <= 2048, from 1.5 slots an SM: n = 2000, p = 0.5, k = 2, pop 256 2185 -> 2287, pop 1024 6737 -> 7456 (pop 160
+//     2120 -> 2100); k = 3, pop 1024 8407 -> 9064 (pop 222 2842 -> 2829); k = 4 and 5 below 90 vertices a unit stay
+//     (n = 2000, p = 0.5, k = 5, pop 320 5272 -> 4924), above p = 0.1, k = 4, pop 512 5728 -> 5987.
+//   k > 8, n <= 1024, from one slot an SM: n = 300, k = 32, pop 512 1496 -> 2074; n = 600, k = 20, pop 256 1956 -> 2220.
+//     Windows are as fast again at pop 512 from n = 450 for k <= 12 (1.01), n = 550 for k <= 16 (1.04) and n = 1000 for more
+//     clusters (k = 20 1.06, k = 32 0.98), n = 900 for k = 64 (1.30: one slot's counters fill an SM).
+// And for k > 56, 1300 < n <= 1600 the incremental form's counters fit shared memory while the windows' do not: n = 1500,
+// k = 64, pop 128 5335 -> 5582, a batch of 16 such instances 82.6 -> 93.0 ms.
+bool PreferWindow(int n, int k, int64_t edges, bool rows_in_smem, int slots, int sms) {
   const double p = n > 1 ? 2.0 * (double)edges / ((double)n * (n - 1)) : 0.0;
   const double width = 2.8 * std::sqrt(std::max(0.0, n * p * (1.0 - p) / k));
-  if (k <= 8) return !rows_in_smem && n <= 1150.0 * width;
-  return n <= 1024 || (n <= 2200.0 * width && (k <= 32 || width >= 4.0));
+  if (k <= 8) {
+    if (rows_in_smem || n > 1150.0 * width) return false;
+    return k > 5 || n > 2048 || 2ll * slots <= 3ll * sms || (k >= 4 && n <= 90.0 * width);
+  }
+  if (n <= 1024) return slots <= sms || k * n >= 57000 || n >= (k <= 12 ? 450 : k <= 16 ? 550 : 1000);
+  if (k > 56 && n > 1300 && n <= 1600) return false;
+  return n <= 2200.0 * width && (k <= 32 || width >= 4.0);
 }
 
 // The same for the wide path (32767 < n <= 65536), whose windows hold up to 4096 members at k <= 4.  us a move (B200, the
@@ -273,7 +289,10 @@ size_t NextBytes(const Plan& plan, int n, int k, int ld, int pop) {
   return (size_t)pop * ld * (plan.small_k ? std::max(k, SmallKLanes(k)) : k) * (plan.wide ? 4 : 2);
 }
 
-Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop, int64_t edges) {
+// `slots`: the slots whose descents share the device (the population, or what a batch or server runs together); windows =
+// false: never the windowed descent.
+Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop, int64_t edges, int slots,
+              bool windows = true) {
   Plan p;
   p.wide = n > CCB_MAX_VERTICES_NARROW || ls_kernel == CCB_LS_WIDE;
   p.threads = DescentThreads(n, p.wide);
@@ -347,7 +366,8 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
     p.threads = sk.threads;
     p.smem_bytes = sk.smem_bytes;
   }
-  if (!p.wide && k >= 2 && ls_kernel == CCB_LS_AUTO && PreferWindow(n, k, edges, p.small_k && p.sk.smem_rows)) {
+  if (!p.wide && k >= 2 && ls_kernel == CCB_LS_AUTO && windows &&
+      PreferWindow(n, k, edges, p.small_k && p.sk.smem_rows, slots, dev.sms)) {
     SmallKPlan w;
     if (PlanWindow(w, n, k, false, limit)) {
       p.sk = w;
@@ -359,7 +379,8 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
       p.smem_bytes = w.smem_bytes;
     }
   }
-  if (p.wide && n <= kMaxVerticesIncrementalWide && k >= 2 && ls_kernel == CCB_LS_AUTO && PreferWindowWide(n, k, edges)) {
+  if (p.wide && n <= kMaxVerticesIncrementalWide && k >= 2 && ls_kernel == CCB_LS_AUTO && windows &&
+      PreferWindowWide(n, k, edges)) {
     // uint16 counters: exact while every degree < 65536
     SmallKPlan w;
     if (PlanWindow(w, n, k, true, limit)) {
@@ -689,7 +710,8 @@ void SetRebuild(ccb_solver& s, int kind) {
   if (!s.tensor && s.masks == nullptr) s.Alloc(s.masks, (size_t)s.pop * s.k * s.graph->pitch);
 }
 
-ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool plain = true) {
+// plain: iterated by the plain path; else by the batched engine, beside `slots` others (MakePlan).
+ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool plain = true, int slots = 0) {
   TraceRange trace_range("ccb.solver.create");
   std::unique_ptr<ccb_solver> s(new ccb_solver());
   s->graph = g;
@@ -702,7 +724,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   s->ld = std::max(32, (g->n + 31) / 32 * 32);
   s->ls_kernel = ls_kernel;
   s->plain = plain;
-  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges);
+  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges, plain ? pop : slots);
   // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
   s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
   PlanSmem16(*s);
@@ -1410,6 +1432,11 @@ void EnqueueIteration(WorkLists& w, const BatchEntry* d_entries, int count, int3
   CCB_CUDA(LaunchBatchAdvance(d_entries, count, d_active, d_stops, st));
 }
 
+// Instances whose batched descent without windows runs several slots an SM: PreferWindow compares by how many run
+// together.  (Batched register descents, k <= 8, were slower than windows at any load: n = 2000, k = 2, 16 instances of
+// pop 128, 5 iterations 39.7 -> 35.9 ms.)
+bool SharesSms(int n, int k) { return k > 8 && n <= 1024; }
+
 void PrepareBatch(ccb_batch& b) {
   if (b.prepared) return;
   if (b.stream == nullptr) CCB_CUDA(cudaStreamCreateWithFlags(&b.stream, cudaStreamNonBlocking));
@@ -1417,10 +1444,16 @@ void PrepareBatch(ccb_batch& b) {
   b.batched.clear();
   std::vector<BatchEntry> entries;
   std::vector<const ccb_solver*> solvers;
+  long long together = 0;  // the flow engine's kernels run one slot an SM with or without windows
+  for (const ccb_batch::Instance& in : b.inst) {
+    if (b.engine == CCB_BATCH_LOCKSTEP && SharesSms(in.graph->n, in.params.k)) together += in.params.population;
+  }
+  const int slots = (int)std::min<long long>(together, INT32_MAX);
   for (size_t i = 0; i < b.inst.size(); ++i) {
     ccb_batch::Instance& in = b.inst[i];
     if (in.graph->n == 0) continue;
-    in.solver.reset(MakeSolver(in.graph, in.params.k, in.params.population, CCB_LS_AUTO, false));
+    in.solver.reset(MakeSolver(in.graph, in.params.k, in.params.population, CCB_LS_AUTO, false,
+                               SharesSms(in.graph->n, in.params.k) ? slots : 0));
     const Plan& pl = in.solver->plan;
     in.batched = !pl.wide && (pl.small_k || pl.incremental);
     if (!in.batched) continue;
@@ -1706,10 +1739,10 @@ size_t RequestBytes(const ccb_server& sv, uint32_t n, const ccb_params& p) {
   const int ld = std::max(32, ((int)n + 31) / 32 * 32);
   const int kpad = (p.k + 3) / 4 * 4;
   // The descent, and with it its scratch, depends on the graph's density, not known before a generated graph's
-  // admission: the larger of both.
-  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0);
+  // admission, and on the load: the larger of both.
+  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0, 0, false);
   const Plan dense = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population,
-                              (int64_t)n * (n - 1) / 4);
+                              (int64_t)n * (n - 1) / 4, 0);
   const size_t labels = (size_t)p.population * ld;
   const size_t gb = plan.wide ? 4 : 2;
   const size_t next = std::max(NextBytes(plan, (int)n, p.k, ld, p.population),
@@ -1831,8 +1864,21 @@ bool BatchedKernelsTake(const ccb_server& sv, const ccb_server::Request& r) {
   const int pitch = std::max(4, (words + 3) / 4 * 4);
   const int ld = std::max(32, ((int)r.n + 31) / 32 * 32);
   const Plan pl = MakePlan((int)r.n, pitch, r.params.k, ld, (r.params.k + 3) / 4 * 4, CCB_LS_AUTO, sv.device,
-                           r.params.population, 0);
+                           r.params.population, 0, 0);
   return !pl.wide && (pl.small_k || pl.incremental);
+}
+
+// The slots that run beside a request's in its lane: those admitted and those queued for it.
+int LaneSlots(const ccb_server& sv, const ccb_server::Request& r) {
+  if (!SharesSms((int)r.n, r.params.k)) return 0;
+  long long slots = r.params.population;
+  for (const ccb_server::Active& a : sv.lanes[ccb_server::LaneOf(r.n)].active) {
+    if (SharesSms((int)a.req.n, a.req.params.k)) slots += a.req.params.population;
+  }
+  for (const ccb_server::Request& q : sv.queue) {
+    if (SharesSms((int)q.n, q.params.k)) slots += q.params.population;
+  }
+  return (int)std::min<long long>(slots, INT32_MAX);
 }
 
 // Admits queued requests (FIFO) while the device-memory budget and the active-slot cap allow; a request
@@ -1869,7 +1915,7 @@ void Admit(ccb_server& sv) {
         Finish(sv, a, r0, {});
         continue;
       }
-      a.solver.reset(MakeSolver(a.graph.get(), q.params.k, q.params.population, CCB_LS_AUTO, false));
+      a.solver.reset(MakeSolver(a.graph.get(), q.params.k, q.params.population, CCB_LS_AUTO, false, LaneSlots(sv, q)));
       const Plan& pl = a.solver->plan;
       if (pl.wide || !(pl.small_k || pl.incremental)) {
         CCB_CUDA(cudaStreamSynchronize(sv.stream));  // the graph is complete before another stream reads it
@@ -2377,7 +2423,7 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
   // the narrow descent depends on the density: another one than the cached solver's needs other buffers
   const auto same_descent = [&] {
     const ccb_solver& s = *c.solver;
-    return MakePlan(s.n, s.graph->pitch, k, s.ld, s.kpad, ls_kernel, s.device, pop, (int64_t)edges).sk.window ==
+    return MakePlan(s.n, s.graph->pitch, k, s.ld, s.kpad, ls_kernel, s.device, pop, (int64_t)edges, pop).sk.window ==
            s.plan.sk.window;
   };
   if (c.solver && c.device == device && c.n == n && c.k == k && c.pop == pop && c.ls == ls_kernel && same_descent()) {

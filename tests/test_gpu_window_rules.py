@@ -47,3 +47,39 @@ def test_ties_match_oracle(ccb, oracle, cuda_device, n, parts, k, p_in, p_out):
     got = solver.pbils(ccb.PbilsParams(**p))
     assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
     assert np.array_equal(got.labels, want.labels)
+
+
+# Populations that fill the SMs more than once, where other descents keep several slots on an SM: the route follows the load
+# (n <= 2048, k <= 5 and n <= 1024, k > 8), and both sides of each line follow the oracle
+@pytest.mark.parametrize("n,k,pop,density,windowed", [
+    (1400, 2, 160, 0.5, True), (1400, 2, 240, 0.5, False), (1400, 3, 240, 0.5, False), (1400, 4, 300, 0.5, True),
+    (1400, 5, 300, 0.1, False), (1400, 6, 300, 0.1, True),
+    (200, 9, 148, 0.3, True), (200, 9, 150, 0.3, False), (460, 12, 150, 0.3, True), (460, 16, 150, 0.3, False),
+    (560, 16, 150, 0.3, True), (560, 17, 150, 0.3, False), (900, 64, 150, 0.3, True), (850, 64, 150, 0.3, False),
+    (1400, 60, 8, 0.3, False)])
+def test_route_follows_the_load(ccb, oracle, cuda_device, n, k, pop, density, windowed):
+    bits, edges = oracle.erdos_renyi(n, density, n + k)
+    p = dict(k=k, population=pop, iterations=1, early_stop=10, seed=4)
+    solver = ccb.Solver(ccb.DeviceGraph(ccb.Graph(n, bits, edges)), ccb.PbilsParams(**p))
+    assert solver.describe().startswith("windowed") == windowed, solver.describe()
+    got = solver.pbils(ccb.PbilsParams(**p))
+    want = oracle.pbils(bits, edges, make_params(**p))
+    assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+    assert np.array_equal(got.labels, want.labels)
+    one = ccb.SolveGpu(ccb.Graph(n, bits, edges), ccb.PbilsParams(**p))
+    assert one.objective == want.objective and np.array_equal(one.labels, want.labels)
+
+
+@pytest.mark.parametrize("engine,count,windowed", [("lockstep", 2, True), ("lockstep", 6, False), ("flow", 6, True)])
+def test_batched_route_follows_the_load(ccb, cuda_device, engine, count, windowed):
+    batch = ccb.Batch(engine=engine)
+    p = [ccb.PbilsParams(k=20, population=60, iterations=3, early_stop=10, seed=s) for s in range(count)]
+    graphs = [ccb.DeviceGraph.erdos_renyi(300, 0.3, 50 + i) for i in range(count)]
+    ids = [batch.add(g, q) for g, q in zip(graphs, p)]
+    batch.run()
+    assert batch.describe().startswith("windowed") == windowed, batch.describe()
+    for i, g, q in zip(ids, graphs, p):
+        got, want = batch.result(i), ccb.Solver(g, q).pbils(q)
+        assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+        assert np.array_equal(got.labels, want.labels)
+    batch.close()
