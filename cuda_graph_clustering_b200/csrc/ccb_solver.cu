@@ -280,6 +280,23 @@ bool PreferWindowWide(int n, int k, int64_t edges) {
   return n <= (k == 2 ? 500.0 : k == 3 ? 1500.0 : 4000.0) * width;
 }
 
+// Whether open twins by the thousand keep a graph from the windows: a move raises the gains of the moved vertex's twins, the
+// rest of them may then be better than any member, and the window ends.  On a complete multipartite graph the share of such
+// pairs is 1 / parts.  us a pass (B200, pop 128, 1 iteration), without windows -> windowed:
+//   two parts, k <= 8, also nearly complete ones: n = 16000, k = 3 1348 -> 2623, with 0.05 % of the pairs flipped 49290 ->
+//     61085; n = 3000, k = 4 432 -> 684 and 1741 -> 4115, with 0.4 % flipped 3151 -> 3736, with 2 % windows are faster.  More
+//     clusters: n = 6000, k = 40 faster as a complete graph (36840 -> 12260), slower with 0.05 % flipped (84439 -> 107937);
+//   more parts, complete, k = 2 to 4 and over 1700 (k - 1) vertices each: n = 16000, 3 parts, k = 2 53210 -> 87624, k = 4 81812 ->
+//     97831, 4 parts, k = 3 69893 -> 76011; but n = 6000, 3 parts, k = 3, n = 16000, 8 parts, k = 2 and any with 0.05 %
+//     flipped (n = 16000, 3 parts, k = 3 69727 -> 37650) are faster windowed;
+//   wide: two parts, k = 2, 3: n = 36000, k = 3 2368 -> 3601, k = 4 17399 -> 5882; 3 parts, k = 2, n = 60000 384.7 -> 694.2 ms,
+//     n = 36000 153.1 -> 134.3 ms.
+bool SlowTies(int n, int k, const OpenTwins& twins, bool wide) {
+  if (twins.near >= 0.4) return k <= (wide ? 3 : 8);
+  if (twins.exact < 0.22) return false;
+  return wide ? k == 2 && n * twins.exact > 15000.0 : k <= 4 && n * twins.exact > 1700.0 * (k - 1);
+}
+
 // Bytes of the population's descent scratch in global memory (the slots' rows of `next`); 0 when the state is in
 // shared memory or registers.
 size_t NextBytes(const Plan& plan, int n, int k, int ld, int pop) {
@@ -291,8 +308,8 @@ size_t NextBytes(const Plan& plan, int n, int k, int ld, int pop) {
 
 // `slots`: the slots whose descents share the device (the population, or what a batch or server runs together); windows =
 // false: never the windowed descent.
-Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop, int64_t edges, int slots,
-              bool windows = true) {
+Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop, int64_t edges,
+              const OpenTwins& twins, int slots, bool windows = true) {
   Plan p;
   p.wide = n > CCB_MAX_VERTICES_NARROW || ls_kernel == CCB_LS_WIDE;
   p.threads = DescentThreads(n, p.wide);
@@ -367,7 +384,7 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
     p.smem_bytes = sk.smem_bytes;
   }
   if (!p.wide && k >= 2 && ls_kernel == CCB_LS_AUTO && windows &&
-      PreferWindow(n, k, edges, p.small_k && p.sk.smem_rows, slots, dev.sms)) {
+      PreferWindow(n, k, edges, p.small_k && p.sk.smem_rows, slots, dev.sms) && !SlowTies(n, k, twins, false)) {
     SmallKPlan w;
     if (PlanWindow(w, n, k, false, limit)) {
       p.sk = w;
@@ -380,7 +397,7 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
     }
   }
   if (p.wide && n <= kMaxVerticesIncrementalWide && k >= 2 && ls_kernel == CCB_LS_AUTO && windows &&
-      PreferWindowWide(n, k, edges)) {
+      PreferWindowWide(n, k, edges) && !SlowTies(n, k, twins, true)) {
     // uint16 counters: exact while every degree < 65536
     SmallKPlan w;
     if (PlanWindow(w, n, k, true, limit)) {
@@ -724,7 +741,8 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   s->ld = std::max(32, (g->n + 31) / 32 * 32);
   s->ls_kernel = ls_kernel;
   s->plain = plain;
-  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges, plain ? pop : slots);
+  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges, g->twins,
+                     plain ? pop : slots);
   // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
   s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
   PlanSmem16(*s);
@@ -1740,9 +1758,10 @@ size_t RequestBytes(const ccb_server& sv, uint32_t n, const ccb_params& p) {
   const int kpad = (p.k + 3) / 4 * 4;
   // The descent, and with it its scratch, depends on the graph's density, not known before a generated graph's
   // admission, and on the load: the larger of both.
-  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0, 0, false);
+  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0, OpenTwins(), 0,
+                             false);
   const Plan dense = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population,
-                              (int64_t)n * (n - 1) / 4, 0);
+                              (int64_t)n * (n - 1) / 4, OpenTwins(), 0);
   const size_t labels = (size_t)p.population * ld;
   const size_t gb = plan.wide ? 4 : 2;
   const size_t next = std::max(NextBytes(plan, (int)n, p.k, ld, p.population),
@@ -1864,7 +1883,7 @@ bool BatchedKernelsTake(const ccb_server& sv, const ccb_server::Request& r) {
   const int pitch = std::max(4, (words + 3) / 4 * 4);
   const int ld = std::max(32, ((int)r.n + 31) / 32 * 32);
   const Plan pl = MakePlan((int)r.n, pitch, r.params.k, ld, (r.params.k + 3) / 4 * 4, CCB_LS_AUTO, sv.device,
-                           r.params.population, 0, 0);
+                           r.params.population, 0, OpenTwins(), 0);
   return !pl.wide && (pl.small_k || pl.incremental);
 }
 
@@ -2420,13 +2439,7 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
   int device = 0;
   CCB_CUDA(cudaGetDevice(&device));
   OneCallCache& c = t_cache;
-  // the narrow descent depends on the density: another one than the cached solver's needs other buffers
-  const auto same_descent = [&] {
-    const ccb_solver& s = *c.solver;
-    return MakePlan(s.n, s.graph->pitch, k, s.ld, s.kpad, ls_kernel, s.device, pop, (int64_t)edges, pop).sk.window ==
-           s.plan.sk.window;
-  };
-  if (c.solver && c.device == device && c.n == n && c.k == k && c.pop == pop && c.ls == ls_kernel && same_descent()) {
+  if (c.solver && c.device == device && c.n == n && c.k == k && c.pop == pop && c.ls == ls_kernel) {
     const int words = (int)((n + 31) / 32);
     if (words_per_row < (uint32_t)words) Fail(CCB_ERR_INVALID, "words_per_row < ceil(n / 32)");
     if (bits == nullptr) Fail(CCB_ERR_INVALID, "null bitset");
@@ -2435,6 +2448,15 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
     CCB_CUDA(cudaMemcpy2DAsync(g.bits, g.pitch * sizeof(uint32_t), bits, words_per_row * sizeof(uint32_t),
                                words * sizeof(uint32_t), n, cudaMemcpyHostToDevice, nullptr));
     FinishGraph(g, nullptr);
+    // the windowed descent depends on the density and the ties: a change needs other buffers
+    const ccb_solver& old = *c.solver;
+    const bool windows = MakePlan(old.n, g.pitch, k, old.ld, old.kpad, ls_kernel, old.device, pop, g.edges, g.twins,
+                                  pop).sk.window;
+    if (windows != old.plan.sk.window) {
+      c.solver.reset();
+      c.solver.reset(MakeSolver(&g, k, pop, ls_kernel));
+      return *c.solver;
+    }
     // the plan's k = 2 / 3 wide form depends on the density
     ccb_solver& s = *c.solver;
     s.plan.sparse = s.plan.packed_wide && 2.0 * (double)edges <= (double)n * n / 8.0;

@@ -36,8 +36,9 @@ def test_ties_cost_no_window_a_move(ccb, cuda_device, n, parts, k):
 
 # The same ties against the oracle: closed twins (gains fall together), open twins (they rise), classes of both, with windows
 # of vertex-keyed members (k <= 8), of members in order (k > 8) and of counters in shared memory (k > 32)
-@pytest.mark.parametrize("p_in,p_out", [(1.0, 0.0), (0.0, 1.0)])
-@pytest.mark.parametrize("n,parts,k", [(4000, 2, 3), (5000, 3, 4), (4100, 2, 16), (4200, 2, 40)])
+@pytest.mark.parametrize("n,parts,k,p_in,p_out", [
+    (4000, 2, 3, 1.0, 0.0), (5000, 3, 4, 1.0, 0.0), (4100, 2, 16, 1.0, 0.0), (4200, 2, 40, 1.0, 0.0),
+    (4800, 4, 3, 0.0, 1.0), (5000, 3, 4, 0.0, 1.0), (4100, 2, 16, 0.0, 1.0), (4800, 4, 40, 0.0, 1.0)])
 def test_ties_match_oracle(ccb, oracle, cuda_device, n, parts, k, p_in, p_out):
     bits, edges, _ = oracle.planted(n, parts, False, p_in, p_out, 0.0, 5)
     p = dict(k=k, population=2, iterations=2, early_stop=10, seed=2)
@@ -83,3 +84,33 @@ def test_batched_route_follows_the_load(ccb, cuda_device, engine, count, windowe
         assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
         assert np.array_equal(got.labels, want.labels)
     batch.close()
+
+
+# Open twins: the vertices of one part of a nearly complete multipartite graph.  Two large parts lose by windows (moves raise
+# the gains of the twins), many parts and closed twins (communities) do not; the one-call cache follows.
+@pytest.mark.parametrize("n,parts,k,p_in,p_out,flip,windowed", [
+    (3000, 2, 3, 0.0, 1.0, 0.0, False), (3001, 2, 5, 0.0, 1.0, 0.0005, False), (3000, 2, 12, 0.0, 1.0, 0.0, True),
+    (6000, 3, 2, 0.0, 1.0, 0.0, False), (6000, 3, 3, 0.0, 1.0, 0.0, True), (3000, 2, 3, 0.0, 1.0, 0.05, True),
+    (3000, 8, 2, 0.0, 1.0, 0.0, True), (6000, 3, 2, 0.0, 1.0, 0.0005, True), (3000, 2, 3, 1.0, 0.0, 0.0, True), (36000, 2, 3, 0.0, 1.0, 0.0, False),
+    (36000, 2, 4, 0.0, 1.0, 0.0, True)])
+def test_open_twins_keep_the_other_descents(ccb, oracle, cuda_device, n, parts, k, p_in, p_out, flip, windowed):
+    graph, _ = ccb.DeviceGraph.planted(n, parts, p_in, p_out, flip, 6)
+    p = dict(k=k, population=2, iterations=1, early_stop=10, seed=2)
+    solver = ccb.Solver(graph, ccb.PbilsParams(**p))
+    assert solver.describe().startswith("windowed") == windowed, solver.describe()
+    host = graph.download()
+    want = oracle.pbils(host.bits, host.edges, make_params(**p)) if n < 10000 else \
+        ccb.SolveGpu(host, ccb.PbilsParams(**p, ls_kernel=ccb.LS_WIDE))
+    for got in (solver.pbils(ccb.PbilsParams(**p)), ccb.SolveGpu(host, ccb.PbilsParams(**p))):
+        assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+        assert np.array_equal(got.labels, want.labels)
+
+
+def test_one_call_cache_follows_the_ties(ccb, oracle, cuda_device):
+    p = dict(k=3, population=2, iterations=1, early_stop=10, seed=3)
+    for p_in, p_out in ((0.0, 1.0), (0.6, 0.2), (0.0, 1.0)):
+        bits, edges, _ = oracle.planted(2500, 2, True, p_in, p_out, 0.0, 3)
+        want = oracle.pbils(bits, edges, make_params(**p))
+        got = ccb.SolveGpu(ccb.Graph(2500, bits, edges), ccb.PbilsParams(**p))
+        assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+        assert np.array_equal(got.labels, want.labels)
