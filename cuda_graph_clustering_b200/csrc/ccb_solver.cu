@@ -690,7 +690,8 @@ bool WantTensor(const ccb_solver& s, int kind) {
   return PlanTensorRebuild(t, s.n, s.pop * s.k, s.device.sms, &why);
 }
 
-// Sets the rebuild kind; allocates the one-hot buffer and encodes the tensor maps when the tensor path is on.
+// Sets the rebuild kind; allocates the one-hot buffer and encodes the tensor maps when the tensor path is on, the masks
+// when it is not.  The solver changes once all of it is there: one whose allocation fails stays as it was.
 void SetRebuild(ccb_solver& s, int kind) {
   if (kind != CCB_REBUILD_AUTO && kind != CCB_REBUILD_POPCOUNT && kind != CCB_REBUILD_TENSOR) {
     Fail(CCB_ERR_INVALID, "rebuild kind must be CCB_REBUILD_AUTO, CCB_REBUILD_POPCOUNT or CCB_REBUILD_TENSOR");
@@ -699,10 +700,12 @@ void SetRebuild(ccb_solver& s, int kind) {
     Fail(CCB_ERR_INVALID, "the tensor-core rebuild runs on the wide path (int32 G: n > 32767 or --ls-kernel wide) "
                           "with n >= 128");
   }
-  s.rebuild_kind = kind;
   std::unique_ptr<TensorRebuild> t;
   if (WantTensor(s, kind)) {
-    if (s.tensor) return;
+    if (s.tensor) {
+      s.rebuild_kind = kind;
+      return;
+    }
     t.reset(new TensorRebuild());
     const char* why = nullptr;
     PlanTensorRebuild(*t, s.n, s.pop * s.k, s.device.sms, &why);
@@ -723,8 +726,9 @@ void SetRebuild(ccb_solver& s, int kind) {
       CCB_CUDA(EncodeTensorRebuild(*t, s.graph->bits, s.graph->pitch, s.z));
     }
   }
+  if (!t && s.masks == nullptr) s.Alloc(s.masks, (size_t)s.pop * s.k * s.graph->pitch);
   s.tensor = std::move(t);
-  if (!s.tensor && s.masks == nullptr) s.Alloc(s.masks, (size_t)s.pop * s.k * s.graph->pitch);
+  s.rebuild_kind = kind;
 }
 
 // plain: iterated by the plain path; else by the batched engine, beside `slots` others (MakePlan).

@@ -32,6 +32,7 @@ struct Failure {
   do {                                                                                                     \
     const cudaError_t e_ = (call);                                                                         \
     if (e_ != cudaSuccess) {                                                                               \
+      cudaGetLastError(); /* reported here: the next launch's check starts clean */                        \
       throw ::ccb::Failure{CCB_ERR_CUDA, std::string("cuda error at ") + __FILE__ + ":" +                  \
                                              std::to_string(__LINE__) + ": " + cudaGetErrorString(e_)};    \
     }                                                                                                      \
