@@ -575,6 +575,7 @@ struct ccb_solver {
   int n = 0, k = 0, kpad = 0, pop = 0, ld = 0;
   int ls_kernel = 0;
   Plan plan;
+  bool windows_refused = false;  // the rule's windowed descent did not fit the free memory
   std::vector<void*> allocations;
   void* cur_g = nullptr;
   void* next_g = nullptr;
@@ -745,20 +746,27 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   s->ld = std::max(32, (g->n + 31) / 32 * 32);
   s->ls_kernel = ls_kernel;
   s->plain = plain;
-  s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges, g->twins,
-                     plain ? pop : slots);
-  // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
-  s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
-  PlanSmem16(*s);
-
   const size_t labels = (size_t)pop * s->ld;
   const size_t gains = labels * k;
-  const size_t gb = s->GainBytes();
-  const size_t next_bytes = NextBytes(s->plan, g->n, k, s->ld, pop);
-  size_t bytes = 2 * labels + gains * gb + next_bytes + (size_t)pop * s->kpad * 4 + 2 * pop * 8 +
-                 (size_t)pop * k * g->pitch * 4 + 2 * (size_t)pop * 4 + s->ld + sizeof(Control);
+  size_t next_bytes = 0, bytes = 0;
+  const auto plan = [&](bool windows) {
+    s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges, g->twins,
+                       plain ? pop : slots, windows);
+    // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
+    s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
+    PlanSmem16(*s);
+    next_bytes = NextBytes(s->plan, g->n, k, s->ld, pop);
+    bytes = 2 * labels + gains * s->GainBytes() + next_bytes + (size_t)pop * s->kpad * 4 + 2 * pop * 8 +
+            (size_t)pop * k * g->pitch * 4 + 2 * (size_t)pop * 4 + s->ld + sizeof(Control);
+  };
+  plan(true);
   size_t free_b = 0, total_b = 0;
   CCB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  if (bytes > free_b && s->plan.sk.window) {  // the windows' state in L2 may be in shared memory without them
+    plan(false);
+    s->windows_refused = true;
+  }
+  const size_t gb = s->GainBytes();
   if (bytes > free_b) {
     Fail(CCB_ERR_DEVICE_MEMORY, "run needs " + Mebibytes(bytes) + " of device memory, " + Mebibytes(free_b) + " free");
   }
@@ -2456,7 +2464,7 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
     const ccb_solver& old = *c.solver;
     const bool windows = MakePlan(old.n, g.pitch, k, old.ld, old.kpad, ls_kernel, old.device, pop, g.edges, g.twins,
                                   pop).sk.window;
-    if (windows != old.plan.sk.window) {
+    if (windows != old.plan.sk.window && !(windows && old.windows_refused)) {
       c.solver.reset();
       c.solver.reset(MakeSolver(&g, k, pop, ls_kernel));
       return *c.solver;

@@ -46,3 +46,27 @@ def test_solver_survives_a_rebuild_kind_it_has_no_memory_for(ccb, cuda_device):
     solver.set_rebuild("popcount")
     assert "tcgen05" not in solver.describe()
     _same(solver.pbils(p), want)
+
+
+def test_windows_that_do_not_fit_give_way(ccb, cuda_device):
+    """n = 18000, k = 3: the streamed descent has its state in shared memory, the windowed one 108 KB a slot in L2.  With
+    room for the one and not for the other a solver, and a one-call solve, take the first, with the same result."""
+    p = ccb.PbilsParams(k=3, population=2048, iterations=1, early_stop=5, seed=2)
+    graph = ccb.DeviceGraph.erdos_renyi(18000, 0.1, 3)
+    host = graph.download()
+    solver = ccb.Solver(graph, p)
+    assert solver.describe().startswith("windowed")
+    want = solver.pbils(p)
+    solver.close()
+    ccb.lib().ccb_release_cache()
+    with memory_left(460):
+        solver = ccb.Solver(graph, p)
+        assert not solver.describe().startswith("windowed"), solver.describe()
+        _same(solver.pbils(p), want)
+        solver.close()
+        for _ in range(2):
+            _same(ccb.SolveGpu(host, p), want)
+        ccb.lib().ccb_release_cache()
+    solver = ccb.Solver(graph, p)
+    assert solver.describe().startswith("windowed")
+    solver.close()
