@@ -613,6 +613,7 @@ struct ccb_solver {
     ptr = static_cast<T*>(p);
   }
   size_t GainBytes() const { return plan.wide ? 4 : 2; }
+  size_t MaskBytes() const { return (size_t)pop * k * graph->pitch * 4; }
 
   ~ccb_solver() {
     for (void* p : allocations) cudaFree(p);
@@ -727,7 +728,10 @@ void SetRebuild(ccb_solver& s, int kind) {
       CCB_CUDA(EncodeTensorRebuild(*t, s.graph->bits, s.graph->pitch, s.z));
     }
   }
-  if (!t && s.masks == nullptr) s.Alloc(s.masks, (size_t)s.pop * s.k * s.graph->pitch);
+  if (!t && s.masks == nullptr) {
+    s.Alloc(s.masks, s.MaskBytes() / 4);
+    s.device_bytes += s.MaskBytes();
+  }
   s.tensor = std::move(t);
   s.rebuild_kind = kind;
 }
@@ -757,7 +761,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
     PlanSmem16(*s);
     next_bytes = NextBytes(s->plan, g->n, k, s->ld, pop);
     bytes = 2 * labels + gains * s->GainBytes() + next_bytes + (size_t)pop * s->kpad * 4 + 2 * pop * 8 +
-            (size_t)pop * k * g->pitch * 4 + 2 * (size_t)pop * 4 + s->ld + sizeof(Control);
+            s->MaskBytes() + 2 * (size_t)pop * 4 + s->ld + sizeof(Control);
   };
   plan(true);
   size_t free_b = 0, total_b = 0;
@@ -770,7 +774,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   if (bytes > free_b) {
     Fail(CCB_ERR_DEVICE_MEMORY, "run needs " + Mebibytes(bytes) + " of device memory, " + Mebibytes(free_b) + " free");
   }
-  s->device_bytes = bytes;
+  s->device_bytes = bytes - s->MaskBytes();  // SetRebuild adds what its kind allocates
   s->Alloc(s->cur_lab, labels);
   s->Alloc(s->next_lab, labels);
   uint8_t* cg = nullptr;

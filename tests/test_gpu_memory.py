@@ -1,5 +1,7 @@
 """Calls that run out of device memory: they fail alone, and what was there goes on working."""
 import contextlib
+import ctypes
+import re
 
 import numpy as np
 import pytest
@@ -70,3 +72,17 @@ def test_windows_that_do_not_fit_give_way(ccb, cuda_device):
     solver = ccb.Solver(graph, p)
     assert solver.describe().startswith("windowed")
     solver.close()
+
+
+def test_reported_memory_counts_what_is_allocated(ccb, cuda_device, capfd):
+    """The masks of the popcount rebuild (17.3 MB here) are counted once they are there."""
+    graph = ccb.DeviceGraph.erdos_renyi(4100, 0.2, 3)
+    p = ccb.PbilsParams(k=4, population=8192, iterations=0, verbose=True)
+    solver = ccb.Solver(graph, p)
+    shown = []
+    for kind in ("auto", "popcount"):
+        solver.set_rebuild(kind)
+        solver.pbils(p)
+        ctypes.CDLL(None).fflush(None)
+        shown.append(int(re.search(r"device memory: (\d+) MiB", capfd.readouterr().out).group(1)))
+    assert 16 <= shown[1] - shown[0] <= 18, shown
