@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 
 #include "ccb_streams.cuh"
 
@@ -148,6 +149,8 @@ __device__ __forceinline__ long long BlockSum(long long v, long long* scratch) {
 // batches) share one kernel instance, each with its own need, so the limit must cover the largest.
 template <typename Kernel>
 inline cudaError_t RaiseDynamicSmem(Kernel kernel, size_t bytes) {
+  static std::mutex mutex;  // of this kernel type: what two threads read and set may not interleave
+  std::lock_guard<std::mutex> lock(mutex);
   cudaFuncAttributes attr;
   cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
   if (e != cudaSuccess) return e;

@@ -598,8 +598,9 @@ cudaError_t LaunchTensorRebuild(const TensorRebuild& t, GainT* g, int ld, int n_
   const int columns = count * k;
   if (columns <= 0) return cudaSuccess;
   if (columns > t.z_rows) return cudaErrorInvalidValue;
+  // one limit for every plan: a smaller one set here could come between another thread's limit and its launch
   const cudaError_t attr = cudaFuncSetAttribute(k_rebuild_tensor<LabelT, GainT>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem);
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TensorSmem(kTensorMaxN));
   if (attr != cudaSuccess) return attr;
   TensorArgs a{};
   a.g = g;
