@@ -176,10 +176,15 @@ int Report(int status, const char* message) {
 // vertices and wave of CTAs (256 vertices x 256 columns each), 10 us more of set-up.  n = 20000, k = 16: 106 us against
 // 150 for one labeling, 4290 against 480 for 64; n = 4001, k = 64, 32 labelings: 455 against 83.
 bool PreferTensorRecount(const uint32_t* bits, int n, int words_per_row, int k, int count) {
+  int device = 0, sms = 0;
   if (n < 128 || words_per_row % 4 != 0 || reinterpret_cast<uintptr_t>(bits) % 16 != 0) return false;
   const double words = (n + 31) / 32, columns = (double)count * k;
   if (columns * words * 32 > 1024.0 * 1024 * 1024 || columns > 1 << 24) return false;  // its one-hot scratch
-  const double waves = std::ceil(std::ceil(n / 256.0) * std::ceil(columns / 256) / 148);
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    return false;
+  }
+  const double waves = std::ceil(std::ceil(n / 256.0) * std::ceil(columns / 256) / sms);
   return 10 + waves * std::ceil(words / 4) * 1.25 < n * words * columns / 4.2e6;
 }
 
@@ -243,13 +248,13 @@ int ccb_evaluate_labelings(const uint32_t* bits, uint32_t n, uint32_t words_per_
     return Report(CCB_ERR_INVALID, why);
   }
   if (count == 0) return Report(CCB_OK, "");
-  if (PreferTensorRecount(bits, (int)n, (int)words_per_row, k, count)) {
-    const int status = ccb_evaluate_labelings_tensor(bits, n, words_per_row, edges, k, count, labels, f_out, sizes_out,
-                                                     g_out, stream);
-    if (status != CCB_ERR_DEVICE_MEMORY) return status;  // else by popcount, with a tenth of the scratch
-    cudaGetLastError();
-  }
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (PreferTensorRecount(bits, (int)n, (int)words_per_row, k, count)) {
+    if (RecountTensor(bits, n, words_per_row, edges, k, count, labels, f_out, sizes_out, g_out, st, true, false) == CCB_OK) {
+      return CCB_OK;
+    }
+    cudaGetLastError();  // not enough memory or no contraction here: by popcount, with an eighth of the scratch
+  }
   const int words = (int)((n + 31) / 32);
   const size_t mask_bytes = sizeof(uint32_t) * (size_t)count * k * words;
   uint32_t* masks = nullptr;

@@ -472,18 +472,77 @@ __global__ void __launch_bounds__(kLabelsThreads)
   if (tid == 0 && blockIdx.y == 0) a.intra[slot] = 0;
 }
 
-// f = m + sum_c C(size_c, 2) - intra per labeling (the recount's last step); -1 for a bad label, -2 when the
-// contraction's bounded wait gave up.
-__global__ void k_tensor_finish(const int32_t* sizes, int kpad, const int64_t* intra, const int32_t* bad,
-                                const int32_t* error, int count, int k, long long edges, int64_t* f_out) {
-  const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= count) return;
-  long long pairs = 0;
-  for (int c = 0; c < k; ++c) {
-    const long long sz = sizes[static_cast<size_t>(slot) * kpad + c];
-    pairs += sz * (sz - 1) / 2;
+// What the recount's last step needs to count a labeling again by popcount.
+struct RecountArgs {
+  const uint32_t* bits;
+  int n, words, pitch;
+  const int32_t* labels;  // [count][n]
+  uint32_t* masks;        // scratch: labeling s at s * mask_step words, [k][words]
+  size_t mask_step;
+  int32_t* g;             // [count][k][n], may be null
+};
+
+// One labeling's intra-cluster sum (each pair twice) and, with a.g, its G, by the whole block: the sum in thread 0.
+template <int kThreads>
+__device__ long long RecountByPopcount(const RecountArgs& a, int slot, int k) {
+  constexpr int kWarps = kThreads / kWarp;
+  __shared__ long long s_sum[kWarps];
+  const int lane = threadIdx.x % kWarp;
+  const int warp = threadIdx.x / kWarp;
+  const int32_t* labels = a.labels + static_cast<size_t>(slot) * a.n;
+  uint32_t* masks = a.masks + slot * a.mask_step;
+  for (int w = warp; w < a.words; w += kWarps) {
+    const int v = w * kWarp + lane;
+    const int l = v < a.n ? labels[v] : -1;
+    for (int c = 0; c < k; ++c) {
+      const uint32_t m = __ballot_sync(kAllLanes, l == c);
+      if (lane == 0) masks[static_cast<size_t>(c) * a.words + w] = m;
+    }
   }
-  f_out[slot] = *error ? -2 : bad[slot] ? -1 : edges + pairs - intra[slot];
+  __syncthreads();
+  long long own_sum = 0;
+  for (int v = warp; v < a.n; v += kWarps) {
+    const uint32_t* row = a.bits + static_cast<size_t>(v) * a.pitch;
+    const int own = labels[v];
+    for (int c = 0; c < k; ++c) {
+      int common = 0;
+      for (int w = lane; w < a.words; w += kWarp) common += __popc(row[w] & masks[static_cast<size_t>(c) * a.words + w]);
+      common = __reduce_add_sync(kAllLanes, common);
+      if (lane == 0) {
+        if (a.g != nullptr) a.g[(static_cast<size_t>(slot) * k + c) * a.n + v] = common;
+        if (own == c) own_sum += common;
+      }
+    }
+  }
+  return BlockSum<kWarps>(own_sum, s_sum);
+}
+
+// f = m + sum_c C(size_c, 2) - intra per labeling (the recount's last step); -1 for a bad label.  When the contraction's
+// bounded wait gave up: with a.bits null -2, else each block counts its labelings again, slowly, over the one-hot scratch.
+constexpr int kFinishThreads = 128;
+__global__ void __launch_bounds__(kFinishThreads)
+    k_tensor_finish(const int32_t* sizes, int kpad, const int64_t* intra, const int32_t* bad, const int32_t* error, int count,
+                    int k, long long edges, int64_t* f_out, RecountArgs a) {
+  const int first = blockIdx.x * kFinishThreads;
+  const int slot = first + threadIdx.x;
+  const auto objective = [&](int s, long long own) {
+    long long pairs = 0;
+    for (int c = 0; c < k; ++c) {
+      const long long sz = sizes[static_cast<size_t>(s) * kpad + c];
+      pairs += sz * (sz - 1) / 2;
+    }
+    return bad[s] ? -1ll : edges + pairs - own;
+  };
+  if (*error == 0) {
+    if (slot < count) f_out[slot] = objective(slot, intra[slot]);
+  } else if (a.bits == nullptr) {
+    if (slot < count) f_out[slot] = -2;
+  } else {
+    for (int s = first; s < min(count, first + kFinishThreads); ++s) {
+      const long long own = RecountByPopcount<kFinishThreads>(a, s, k);
+      if (threadIdx.x == 0) f_out[s] = objective(s, own);
+    }
+  }
 }
 
 using EncodeTiledFn = PFN_cuTensorMapEncodeTiled_v12000;
@@ -631,15 +690,9 @@ template cudaError_t LaunchTensorRebuild<uint8_t, int32_t>(const TensorRebuild&,
                                                            const uint8_t*, int, int64_t*, int32_t*, const Control*,
                                                            cudaStream_t);
 
-}  // namespace ccb
-
-using namespace ccb;
-
-extern "C" {
-
-int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k,
-                                  int32_t count, const int32_t* labels, int64_t* f_out, int32_t* sizes_out,
-                                  int32_t* g_out, void* stream) {
+int RecountTensor(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k, int32_t count,
+                  const int32_t* labels, int64_t* f_out, int32_t* sizes_out, int32_t* g_out, cudaStream_t st, bool recover,
+                  bool gave_up) {
   auto report = [](int status, const std::string& message) {
     SetLastError(message);
     return status;
@@ -661,7 +714,6 @@ int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t wor
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return report(CCB_ERR_CUDA, cudaGetErrorString(e));
   if (!PlanTensorRebuild(t, (int)n, count * k, sms, &why)) return report(CCB_ERR_INVALID, why);
-  const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int kpad = (k + 3) / 4 * 4;
   const size_t z_bytes = (size_t)t.z_rows * t.kz;
   const size_t sizes_bytes = sizes_out ? 0 : (size_t)count * kpad * 4;
@@ -680,7 +732,7 @@ int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t wor
     return report(CCB_ERR_CUDA, cudaGetErrorString(err));
   };
   if ((e = cudaMemsetAsync(z + (size_t)count * k * t.kz, 0, z_bytes - (size_t)count * k * t.kz, st)) != cudaSuccess ||
-      (e = cudaMemsetAsync(error, 0, 4, st)) != cudaSuccess) {
+      (e = cudaMemsetAsync(error, gave_up ? 1 : 0, 4, st)) != cudaSuccess) {
     return fail(e);
   }
   if ((e = EncodeTensorRebuild(t, bits, (int)words_per_row, z)) != cudaSuccess) return fail(e);
@@ -691,11 +743,36 @@ int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t wor
                                         st)) != cudaSuccess) {
     return fail(e);
   }
-  k_tensor_finish<<<(count + 127) / 128, 128, 0, st>>>(sizes, sizes_ld, intra, bad, error, count, k, (long long)edges,
-                                                       f_out);
+  // a labeling's k one-hot rows hold its k masks: kz >= 32 words bytes each
+  const RecountArgs again{recover ? bits : nullptr, (int)n, t.words, (int)words_per_row, labels,
+                          reinterpret_cast<uint32_t*>(z), (size_t)k * t.kz / 4, g_out};
+  k_tensor_finish<<<(count + kFinishThreads - 1) / kFinishThreads, kFinishThreads, 0, st>>>(
+      sizes, sizes_ld, intra, bad, error, count, k, (long long)edges, f_out, again);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
   cudaFreeAsync(buf, st);
   return report(CCB_OK, "");
+}
+
+}  // namespace ccb
+
+using namespace ccb;
+
+extern "C" {
+
+int ccb_evaluate_labelings_tensor(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k,
+                                  int32_t count, const int32_t* labels, int64_t* f_out, int32_t* sizes_out,
+                                  int32_t* g_out, void* stream) {
+  return RecountTensor(bits, n, words_per_row, edges, k, count, labels, f_out, sizes_out, g_out,
+                       static_cast<cudaStream_t>(stream), false, false);
+}
+
+// Not in ccb.h: the contraction that ccb_evaluate_labelings takes, with its wait marked as given up from the start, so that
+// a test sees the labelings counted again without making a kernel wait.
+int ccb_test_recount_gave_up(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k,
+                             int32_t count, const int32_t* labels, int64_t* f_out, int32_t* sizes_out, int32_t* g_out,
+                             void* stream) {
+  return RecountTensor(bits, n, words_per_row, edges, k, count, labels, f_out, sizes_out, g_out,
+                       static_cast<cudaStream_t>(stream), true, true);
 }
 
 }  // extern "C"

@@ -43,6 +43,13 @@ struct Failure {
 cudaError_t ScratchAlloc(void** out, size_t bytes, cudaStream_t st);
 void ScratchTrim();
 
+// A recount as one contraction on the tensor cores (ccb_rebuild_tensor.cu; arguments of ccb_evaluate_labelings_tensor).
+// recover: labelings whose contraction gave up waiting are counted again instead of marked by f = -2; gave_up: act as if it
+// had.  A status other than CCB_OK means that the outputs may be incomplete.
+int RecountTensor(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k, int32_t count,
+                  const int32_t* labels, int64_t* f_out, int32_t* sizes_out, int32_t* g_out, cudaStream_t st, bool recover,
+                  bool gave_up);
+
 [[noreturn]] inline void Fail(int status, const std::string& message) { throw Failure{status, message}; }
 
 template <typename F>

@@ -265,7 +265,9 @@ void ccb_server_destroy(ccb_server* server);
  * sizes_out [count][k] and g_out [count][k][n] (int32, cluster-major) may be NULL.  A labeling with a
  * label outside [0, k) gets f = -1.  Scratch (count * k * ceil(n/32) mask words) is taken from a
  * stream-ordered pool for the call.  Large batches over 16-byte aligned rows run as the contraction of
- * ccb_evaluate_labelings_tensor (the same outputs).  Asynchronous on `stream`. */
+ * ccb_evaluate_labelings_tensor (the same outputs, eight times the scratch and at most about 1 GiB) where that
+ * memory can be had; labelings whose contraction gives up its bounded wait are counted again by popcount, so f is
+ * never -2 here.  Asynchronous on `stream`. */
 int ccb_evaluate_labelings(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint64_t edges, int32_t k,
                            int32_t count, const int32_t* labels, int64_t* f_out, int32_t* sizes_out,
                            int32_t* g_out, void* stream);
