@@ -1,6 +1,8 @@
 // Device recount of labelings: objective f, cluster sizes and G = A*Z for a batch of labelings of one graph.
 // This is the GPU form of the reference's post-solve recount ObjectiveBitwise (src/cc_pbils_cpu.cpp:25-53,
 // run by the CLI at include/cc_cli.hpp:337-343) and of State::Rebuild (src/cc_pbils_cpu.cpp:74-95).
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -8,6 +10,7 @@
 #include <cstdint>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 
 #include "ccb.h"
 #include "ccb_device.cuh"
@@ -188,24 +191,40 @@ bool PreferTensorRecount(const uint32_t* bits, int n, int words_per_row, int k, 
   return 10 + waves * std::ceil(words / 4) * 1.25 < n * words * columns / 4.2e6;
 }
 
-constexpr int kScratchMaxDevices = 64;
-constexpr uint64_t kScratchKept = 64ull << 20;  // bytes a device's pool keeps between calls
+constexpr uint64_t kScratchKept = 64ull << 20;  // bytes a context's pool keeps between calls
 std::mutex g_scratch_mutex;
-cudaMemPool_t g_scratch_pool[kScratchMaxDevices] = {};
+std::unordered_map<unsigned long long, cudaMemPool_t> g_scratch_pools;  // by context
+
+// The current context's id, unique for the life of the process (a device reset ends a context and its pools, and the next
+// one has another id); 0 when there is none or the driver cannot tell.
+unsigned long long CurrentContext() {
+  using GetId = PFN_cuCtxGetId_v12000;
+  static const GetId get_id = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const bool found = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<GetId>(p) : nullptr;
+  }();
+  unsigned long long id = 0;
+  return get_id != nullptr && get_id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
 
 }  // namespace
 
 // The default pool gives its memory back at every synchronisation, so each recount mapped its scratch anew (0.2 ms, up to
-// several on a busy host).  A pool of our own per device keeps up to kScratchKept; ccb_release_cache trims it.  Stream
+// several on a busy host).  A pool of our own per context keeps up to kScratchKept; ccb_release_cache trims it.  Stream
 // ordered and thread safe like the default pool, which serves captures and devices without pool support.
 cudaError_t ScratchAlloc(void** out, size_t bytes, cudaStream_t st) {
   int device = 0;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   cudaMemPool_t pool = nullptr;
-  if (cudaGetDevice(&device) == cudaSuccess && device < kScratchMaxDevices &&
-      cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+  unsigned long long context = 0;
+  if (cudaGetDevice(&device) == cudaSuccess && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+      capture == cudaStreamCaptureStatusNone && (context = CurrentContext()) != 0) {
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (g_scratch_pool[device] == nullptr) {
+    cudaMemPool_t& kept_pool = g_scratch_pools[context];
+    if (kept_pool == nullptr) {
       cudaMemPoolProps props{};
       props.allocType = cudaMemAllocationTypePinned;
       props.handleTypes = cudaMemHandleTypeNone;
@@ -214,13 +233,13 @@ cudaError_t ScratchAlloc(void** out, size_t bytes, cudaStream_t st) {
       uint64_t kept = kScratchKept;
       if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
         if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept) == cudaSuccess) {
-          g_scratch_pool[device] = pool;
+          kept_pool = pool;
         } else {
           cudaMemPoolDestroy(pool);
         }
       }
     }
-    pool = g_scratch_pool[device];
+    pool = kept_pool;
   }
   if (pool != nullptr && cudaMallocFromPoolAsync(out, bytes, pool, st) == cudaSuccess) return cudaSuccess;
   cudaGetLastError();  // what failed above is tried again below
@@ -228,10 +247,10 @@ cudaError_t ScratchAlloc(void** out, size_t bytes, cudaStream_t st) {
 }
 
 void ScratchTrim() {
+  const unsigned long long context = CurrentContext();
   std::lock_guard<std::mutex> lock(g_scratch_mutex);
-  for (cudaMemPool_t pool : g_scratch_pool) {
-    if (pool != nullptr) cudaMemPoolTrimTo(pool, 0);
-  }
+  const auto it = g_scratch_pools.find(context);
+  if (it != g_scratch_pools.end() && it->second != nullptr) cudaMemPoolTrimTo(it->second, 0);
   cudaGetLastError();
 }
 

@@ -93,7 +93,8 @@ int ccb_neighborhood_solve(const uint32_t* bits, uint32_t n, uint32_t words_per_
  * population and ls_kernel: a repeated solve then pays the bitset upload, not the allocations.  No
  * counterpart in the reference, whose calls allocate and free everything (cuda/cc_pbils_gpu.cu:105-122).
  * ccb_release_cache frees the calling thread's buffers; they are also freed when the thread exits.  It also gives
- * back the recounts' scratch memory (at most 64 MiB per device is kept between calls). */
+ * back the recounts' scratch memory on the current device (at most 64 MiB per device is kept between calls).  The
+ * one-call buffers do not outlive a cudaDeviceReset: release them before one (recounts need nothing before it). */
 void ccb_release_cache(void);
 
 /* ---- device-resident graphs and reusable solvers ----------------------------------------------
