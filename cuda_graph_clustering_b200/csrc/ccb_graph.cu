@@ -24,27 +24,26 @@ namespace {
 
 constexpr int kGenWarps = 8;
 
-constexpr int kDegreeThreads = 256;
 constexpr int kTwinSamples = 64;
 constexpr int kTwinPairs = kTwinSamples * (kTwinSamples - 1) / 2;
-constexpr int kTwinBlocks = (kTwinPairs + kDegreeThreads / 32 - 1) / (kDegreeThreads / 32);
+constexpr int kDegreeThreads = 256;
 
-// Degrees, a thread per vertex; the blocks past them look at the pairs among kTwinSamples vertices, a warp each, and add
-// open twins to counts[0] (exact) and counts[1] (exact or nearly).  Moving such a vertex raises the gains of all its twins:
-// the kind of tie that the windowed descent is slow on.
-__global__ void __launch_bounds__(kDegreeThreads) k_graph_degrees(const uint32_t* bits, int n, int words, int pitch,
-                                                                 int32_t* degrees, int32_t* counts) {
-  const int blocks = (n + kDegreeThreads - 1) / kDegreeThreads;
-  if (static_cast<int>(blockIdx.x) < blocks) {
-    const int v = blockIdx.x * kDegreeThreads + threadIdx.x;
-    if (v >= n) return;
-    const uint32_t* row = bits + static_cast<size_t>(v) * pitch;
-    int d = 0;
-    for (int w = 0; w < words; ++w) d += __popc(row[w]);
-    degrees[v] = d;
-    return;
-  }
-  const int pair = (blockIdx.x - blocks) * (kDegreeThreads / 32) + threadIdx.x / 32;
+__global__ void __launch_bounds__(kDegreeThreads)
+    k_graph_degrees(const uint32_t* __restrict__ bits, int n, int words, int pitch, int32_t* degrees) {
+  const int v = blockIdx.x * kDegreeThreads + threadIdx.x;
+  if (v >= n) return;
+  const uint32_t* row = bits + static_cast<size_t>(v) * pitch;
+  int d = 0;
+  for (int w = 0; w < words; ++w) d += __popc(row[w]);
+  degrees[v] = d;
+}
+
+// The pairs among kTwinSamples vertices, a warp each: open twins are added to counts[0] (exact) and counts[1] (exact or
+// nearly).  Moving such a vertex raises the gains of all its twins: the kind of tie that the windowed descent is slow on.
+// A launch of its own: beside the degrees, whose threads reuse their rows' lines in L1, it took them 0.3 ms at n = 65536.
+__global__ void __launch_bounds__(kDegreeThreads)
+    k_open_twins(const uint32_t* __restrict__ bits, int n, int words, int pitch, int32_t* counts) {
+  const int pair = blockIdx.x * (kDegreeThreads / 32) + threadIdx.x / 32;
   if (pair >= kTwinPairs) return;
   const int lane = threadIdx.x % 32;
   int i = 1, first = 0;  // samples (i, j), j < i
@@ -182,12 +181,16 @@ void FinishGraph(ccb_graph& g, cudaStream_t stream) {
   const bool sample = g.n > 2048;  // below, windows lose little by them (n = 1400, k = 5 8 %, n = 2400, k = 5 62 %)
   int32_t counts[2] = {g.twins.counted[0], g.twins.counted[1]};
   if (g.n > 0) {
-    const int blocks = (g.n + kDegreeThreads - 1) / kDegreeThreads;
-    k_graph_degrees<<<blocks + (sample ? kTwinBlocks : 0), kDegreeThreads, 0, stream>>>(g.bits, g.n, g.words, g.pitch,
-                                                                                        g.degrees, g.degrees + g.n);
+    k_graph_degrees<<<(g.n + kDegreeThreads - 1) / kDegreeThreads, kDegreeThreads, 0, stream>>>(g.bits, g.n, g.words,
+                                                                                                g.pitch, g.degrees);
     CCB_CUDA(cudaGetLastError());
   }
-  if (sample) CCB_CUDA(cudaMemcpyAsync(counts, g.degrees + g.n, sizeof(counts), cudaMemcpyDeviceToHost, stream));
+  if (sample) {
+    k_open_twins<<<(kTwinPairs * 32 + kDegreeThreads - 1) / kDegreeThreads, kDegreeThreads, 0, stream>>>(
+        g.bits, g.n, g.words, g.pitch, g.degrees + g.n);
+    CCB_CUDA(cudaGetLastError());
+    CCB_CUDA(cudaMemcpyAsync(counts, g.degrees + g.n, sizeof(counts), cudaMemcpyDeviceToHost, stream));
+  }
   CCB_CUDA(cudaStreamSynchronize(stream));
   g.twins.exact = static_cast<double>(counts[0] - g.twins.counted[0]) / kTwinPairs;
   g.twins.near = static_cast<double>(counts[1] - g.twins.counted[1]) / kTwinPairs;
