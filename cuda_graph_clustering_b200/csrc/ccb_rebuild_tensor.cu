@@ -408,10 +408,24 @@ __global__ void __launch_bounds__(256)
 // cluster sizes and their one-hot rows Z in one pass: a block takes `span` vertices of a slot, a thread four of them
 // at a time, whose label bytes and Z words are written whole.
 constexpr int kLabelsThreads = 256;
+
+// Whether the iteration that a rebuild belongs to has been stopped.
+template <typename GainT>
+__device__ __forceinline__ bool RebuildStopped(const RebuildArgs<GainT>& a) {
+  return a.ctl != nullptr && (a.mode == kRebuildPerturb || a.mode == kRebuildCopy) && a.ctl->stop;
+}
+
+// Cluster sizes zeroed for k_labels_z to add to, where several blocks share a slot.
+template <typename GainT>
+__global__ void __launch_bounds__(kLabelsThreads) k_clear_sizes(RebuildArgs<GainT> a, int count) {
+  const int i = blockIdx.x * kLabelsThreads + threadIdx.x;
+  if (i < count && !RebuildStopped(a)) a.cur.sizes[i] = 0;
+}
+
 template <typename GainT>
 __global__ void __launch_bounds__(kLabelsThreads)
     k_labels_z(RebuildArgs<GainT> a, uint8_t* __restrict__ z, int kz, int span) {
-  if (a.ctl != nullptr && (a.mode == kRebuildPerturb || a.mode == kRebuildCopy) && a.ctl->stop) return;
+  if (RebuildStopped(a)) return;
   __shared__ int s_sizes[kMaxK];
   const int slot = blockIdx.x;
   const int tid = threadIdx.x;
@@ -642,9 +656,9 @@ cudaError_t LaunchLabelsZ(const TensorRebuild& t, const RebuildArgs<GainT>& a, i
   const int want = std::max(1, std::min(groups, (2 * sms + count - 1) / count));
   const int span = (groups + want - 1) / want * kTileK;
   const int blocks = (t.kz + span - 1) / span;
-  if (blocks > 1) {
-    const cudaError_t e = cudaMemsetAsync(a.cur.sizes, 0, (size_t)count * a.kpad * sizeof(int32_t), st);
-    if (e != cudaSuccess) return e;
+  if (blocks > 1) {  // a kernel, not a memset: past a stop the population stays as it is
+    const int sizes = count * a.kpad;
+    k_clear_sizes<GainT><<<(sizes + kLabelsThreads - 1) / kLabelsThreads, kLabelsThreads, 0, st>>>(a, sizes);
   }
   k_labels_z<GainT><<<dim3(count, blocks), kLabelsThreads, 0, st>>>(a, t.z, t.kz, span);
   return cudaGetLastError();
@@ -740,7 +754,7 @@ int RecountTensor(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint
   k_build_z<int32_t><<<count, 256, 0, st>>>(labels, label_ld, (int)n, k, t.kz, z, sizes, sizes_ld, intra, bad, nullptr);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
   if ((e = LaunchTensorRebuild<int32_t, int32_t>(t, g_out, (int)n, (int)n, count, k, labels, label_ld, intra, error, nullptr,
-                                        st)) != cudaSuccess) {
+                                                 st)) != cudaSuccess) {
     return fail(e);
   }
   // a labeling's k one-hot rows hold its k masks: kz >= 32 words bytes each

@@ -43,3 +43,13 @@ def test_tensor_memory_loads_wait_in_their_own_statement():
     statements = re.findall(r"asm volatile\((.*?)\);", source("ccb_rebuild_tensor.cu"), flags=re.S)
     loads = [s for s in statements if "tcgen05.ld." in s]
     assert loads and all("tcgen05.wait::ld" in s for s in loads)
+
+
+def test_a_rebuild_past_a_stop_touches_nothing():
+    """The launches of a rebuild that were enqueued before the stop flag was seen run after it: whatever writes to the
+    population is a kernel that looks at the flag, not a memset, which cannot."""
+    text = source("ccb_rebuild_tensor.cu")
+    body = text[text.index("cudaError_t LaunchLabelsZ("):]
+    body = body[:body.index("\n}")]
+    assert "k_labels_z" in body and "cudaMemset" not in body
+    assert text.count("RebuildStopped(a)") >= 2
