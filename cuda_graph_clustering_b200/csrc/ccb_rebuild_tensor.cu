@@ -359,17 +359,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // Z rows, sizes and bad-label flags of the recount's labelings.
-template <typename LabelT>
 __global__ void __launch_bounds__(256)
-    k_build_z(const LabelT* __restrict__ labels, int label_ld, int n, int k, int kz, uint8_t* __restrict__ z,
-              int32_t* __restrict__ sizes, int kpad, int64_t* __restrict__ intra, int32_t* __restrict__ bad,
-              const Control* stop) {
-  if (stop != nullptr && stop->stop) return;
+    k_build_z(const int32_t* __restrict__ labels, int n, int k, int kz, uint8_t* __restrict__ z,
+              int32_t* __restrict__ sizes, int kpad, int64_t* __restrict__ intra, int32_t* __restrict__ bad) {
   __shared__ int s_sizes[kMaxK];
   __shared__ int s_bad;
   const int slot = blockIdx.x;
   const int tid = threadIdx.x;
-  const LabelT* lab = labels + static_cast<size_t>(slot) * label_ld;
+  const int32_t* lab = labels + static_cast<size_t>(slot) * n;
   for (int c = tid; c < k; c += blockDim.x) s_sizes[c] = 0;
   if (tid == 0) s_bad = 0;
   __syncthreads();
@@ -380,12 +377,12 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int u = 4 * i + j;
-      l[j] = u < n ? static_cast<int>(lab[u]) : -1;
+      l[j] = u < n ? lab[u] : -1;
       if (u < n && (l[j] < 0 || l[j] >= k)) {
         s_bad = 1;
         l[j] = -1;
       }
-      if (sizes != nullptr && l[j] >= 0) atomicAdd(&s_sizes[l[j]], 1);
+      if (l[j] >= 0) atomicAdd(&s_sizes[l[j]], 1);
     }
     for (int c = 0; c < k; ++c) {
       rows[static_cast<size_t>(c) * words + i] = static_cast<uint32_t>(l[0] == c) |
@@ -395,12 +392,10 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  if (sizes != nullptr) {
-    for (int c = tid; c < k; c += blockDim.x) sizes[static_cast<size_t>(slot) * kpad + c] = s_sizes[c];
-  }
+  for (int c = tid; c < k; c += blockDim.x) sizes[static_cast<size_t>(slot) * kpad + c] = s_sizes[c];
   if (tid == 0) {
-    if (intra != nullptr) intra[slot] = 0;
-    if (bad != nullptr) bad[slot] = s_bad;
+    intra[slot] = 0;
+    bad[slot] = s_bad;
   }
 }
 
@@ -750,10 +745,9 @@ int RecountTensor(const uint32_t* bits, uint32_t n, uint32_t words_per_row, uint
     return fail(e);
   }
   if ((e = EncodeTensorRebuild(t, bits, (int)words_per_row, z)) != cudaSuccess) return fail(e);
-  const int label_ld = (int)n;
-  k_build_z<int32_t><<<count, 256, 0, st>>>(labels, label_ld, (int)n, k, t.kz, z, sizes, sizes_ld, intra, bad, nullptr);
+  k_build_z<<<count, 256, 0, st>>>(labels, (int)n, k, t.kz, z, sizes, sizes_ld, intra, bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
-  if ((e = LaunchTensorRebuild<int32_t, int32_t>(t, g_out, (int)n, (int)n, count, k, labels, label_ld, intra, error, nullptr,
+  if ((e = LaunchTensorRebuild<int32_t, int32_t>(t, g_out, (int)n, (int)n, count, k, labels, (int)n, intra, error, nullptr,
                                                  st)) != cudaSuccess) {
     return fail(e);
   }
