@@ -102,7 +102,8 @@ __device__ __forceinline__ void DescentRegistersCompact(const DescentArgs<int16_
     }
   }
   const long long start = a.cur.f[w];
-  const int move_budget = static_cast<int>(start);  // f <= n (n - 1) / 2: every move lowers it
+  // every move lowers f, which is at most n (n - 1) / 2 unless the caller's edge count is off by more
+  const int move_budget = static_cast<int>(min(start, 0x7fffffffll));
   int gained = 0;
   int applied = 0;
   int from = 0, to = 0;

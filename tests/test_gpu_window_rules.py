@@ -114,3 +114,14 @@ def test_one_call_cache_follows_the_ties(ccb, oracle, cuda_device):
         got = ccb.SolveGpu(ccb.Graph(2500, bits, edges), ccb.PbilsParams(**p))
         assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
         assert np.array_equal(got.labels, want.labels)
+
+
+# An edge count other than the bitset's shifts every objective by the difference and nothing else, also past 32 bits
+@pytest.mark.parametrize("n,k", [(300, 4), (1023, 8), (1100, 3), (1500, 3), (700, 12)])
+def test_edge_count_beyond_32_bits(ccb, oracle, cuda_device, n, k):
+    bits, edges = oracle.erdos_renyi(n, 0.3, n)
+    p = dict(k=k, population=4, iterations=2, early_stop=10, seed=3)
+    want = oracle.pbils(bits, edges, make_params(**p))
+    got = ccb.SolveGpu(ccb.Graph(n, bits, edges + (3 << 30)), ccb.PbilsParams(**p))
+    assert (got.objective - (3 << 30), got.accepted_moves) == (want.objective, want.accepted_moves)
+    assert np.array_equal(got.labels, want.labels)
