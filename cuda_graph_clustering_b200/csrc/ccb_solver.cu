@@ -236,15 +236,22 @@ constexpr bool kClusterDescent = true;
 
 // Whether the narrow path takes the windowed descent (ccb_descent_window.cuh).  Its windows are long when few vertices
 // share a gain near the best one, so the line is drawn by the width of the gains, about 2.8 sigma with sigma^2 =
-// n p (1 - p) / k the variance of a neighbour count, and the vertices per unit of it (B200, one descent of a slot on
-// G(n, p), us per move, the kernel without windows -> windowed):
-//   k <= 8, at most 1150 vertices a unit:  n = 16000, p = 0.33, k = 3 (190 a unit): 4.5 -> 0.96; n = 32000, p = 0.01,
-//     k = 3 (1110): 5.5 -> 4.6; above it n = 16000, p = 0.01, k = 8 (1280): 4.7 -> 5.5; n = 8000, p = 0.002, k = 3
-//     (1230): 2.5 -> 2.9.  Below n ~ 1280 the bitset fits in shared memory and the register descent needs no row
-//     from L2: n = 1000, p = 0.5, k = 5: 0.42 -> 0.63, against n = 1500, k = 3: 0.68 -> 0.58.
-//   k > 8, at most 2200 a unit:  n = 9001, p = 0.2, k = 24 (230): 11.9 -> 2.9; n = 20000, p = 0.005, k = 9 (2140): 22.9
-//     -> 12.5; up to 1024 vertices all are members and no gain width is needed (n = 1000, p = 0.33, k = 16: 2.2 ->
-//     1.0).  With k > 32 and a width below 4 most keys tie: n = 4000, p = 0.02, k = 64 (width 3.1): 7.5 -> 9.7.
+// n p (1 - p) / k the variance of a neighbour count, and the vertices per unit of it.  Break-even on G(n, p), pop 128 (B200; a
+// pass without windows over one with them, by vertices a unit):
+//   k <= 8, n <= 2048, against the register descent, 40 k:  n = 2040, k = 2 75 1.02, 100 0.97, 450 0.62; k = 5 170 1.03, 220 0.97;
+//     k = 8 280 1.03, 350 0.95.  Below n ~ 1280 its bitset fits in shared memory and it needs no row from L2.
+//   k <= 8, n <= 4096, the same with one slot an SM, 130 + 80 k:  n = 3000, k = 2 280 1.02, 350 0.96; k = 5 450 1.07, 550 0.96; k =
+//     8 750 1.02, 850 0.92 (the flow engine's line is about 70 higher at k = 2: 278 1.12, 439 0.92).
+//   k <= 8, n > 4096, against the streamed descent, 1150 and less below n ~ 8000:  n = 4200, k = 2 800 0.98, k = 4 900 1.01,
+//     n = 7000, k = 2 1000 1.03, 1100 0.95, n = 6000, k = 5 1140 1.19; n = 32000, k = 3 1110 2.15, and past the line, which
+//     could move up there, n = 8000, k = 3 1230 1.10, n = 16000, k = 8 1280 1.79.
+//   k > 8, against the incremental descent, 2200:  n = 9001, p = 0.2, k = 24 (230) 4.5; n = 20000, k = 9 2140 1.68; for k > 20,
+//     1400 < n < 3000 1750:  n = 2000, k = 32 1200 1.04, 1600 0.93, 2150 0.72, n = 2100 1600 1.15, 2150 0.89, n = 1050 2150
+//     1.8.  Up to 1024 vertices all are members and no width is needed (n = 200 to 1000, p = 0.002 to 0.33: 1.03 to 3.9).
+//     With k > 32 and a width below 4 most keys tie: n = 4000, p = 0.02, k = 64 (3.1) 0.90.  For k > 56, 1300 < n <= 1600 the
+//     incremental form's counters fit shared memory while the windows' do not: n = 1500, k = 64 0.96, a batch of 16 such
+//     instances 0.89.
+// ns a move there: n = 16000, p = 0.33, k = 3 4421 -> 828; n = 9001, k = 24 12009 -> 2608; n = 1500, p = 0.5, k = 3 690 -> 565.
 // An SM holds one windowed slot at a time, but two of the register descent at n <= 2048, k <= 5 and two to eight of the
 // incremental one at n <= 1024 (two while k n < 57000: its counters are in shared memory), so the line moves up once the
 // `slots` that run side by side fill the SMs more than once.  us a pass, without windows -> windowed:
@@ -254,30 +261,32 @@ constexpr bool kClusterDescent = true;
 //   k > 8, n <= 1024, from one slot an SM: n = 300, k = 32, pop 512 1496 -> 2074; n = 600, k = 20, pop 256 1956 -> 2220.
 //     Windows are as fast again at pop 512 from n = 450 for k <= 12 (1.01), n = 550 for k <= 16 (1.04) and n = 1000 for more
 //     clusters (k = 20 1.06, k = 32 0.98), n = 900 for k = 64 (1.30: one slot's counters fill an SM).
-// And for k > 56, 1300 < n <= 1600 the incremental form's counters fit shared memory while the windows' do not: n = 1500,
-// k = 64, pop 128 5335 -> 5582, a batch of 16 such instances 82.6 -> 93.0 ms.
 bool PreferWindow(int n, int k, int64_t edges, bool rows_in_smem, int slots, int sms) {
   const double p = n > 1 ? 2.0 * (double)edges / ((double)n * (n - 1)) : 0.0;
   const double width = 2.8 * std::sqrt(std::max(0.0, n * p * (1.0 - p) / k));
   if (k <= 8) {
-    if (rows_in_smem || n > 1150.0 * width) return false;
-    return k > 5 || n > 2048 || 2ll * slots <= 3ll * sms || (k >= 4 && n <= 90.0 * width);
+    if (rows_in_smem) return false;
+    if (n <= 2048) {
+      const bool fills = k <= 5 && 2ll * slots > 3ll * sms;
+      return n <= (fills ? (k >= 4 ? 90.0 : 0.0) : 40.0 * k) * width;
+    }
+    return n <= (n <= 4096 ? 130.0 + 80.0 * k : std::min(1150.0, 0.09 * n + (k == 2 ? 400.0 : k <= 4 ? 550.0 : 700.0))) * width;
   }
   if (n <= 1024) return slots <= sms || k * n >= 57000 || n >= (k <= 12 ? 450 : k <= 16 ? 550 : 1000);
   if (k > 56 && n > 1300 && n <= 1600) return false;
-  return n <= 2200.0 * width && (k <= 32 || width >= 4.0);
+  return n <= (k > 20 && n > 1400 && n < 3000 ? 1750.0 : 2200.0) * width && (k <= 32 || width >= 4.0);
 }
 
-// The same for the wide path (32767 < n <= 65536), whose windows hold up to 4096 members at k <= 4.  us a move (B200, the
-// kernel without windows -> windowed; vertices per unit of gain width in brackets):
-//   k = 2, whose degree-proportional kernel is cheap: G(50001, 0.1) [376] 5.4 -> 2.2, but G(33000, 0.02) [656] 2.2 -> 2.4;
-//   k = 3: G(65536, 0.02) [1130] 8.3 -> 4.2, but G(65536, 0.005) [2250] 4.5 -> 6.2;
-//   k >= 4: G(40000, 0.05), k = 6 [800] 35 -> 3.3; G(40000, 0.01), k = 8 [2030] 39 -> 8.0; G(65536, 0.01), k = 9 [2750]
-//     59 -> 23.
+// The same for the wide path (32767 < n <= 65536), whose windows hold up to 4096 members at k <= 4 (pop 32; without windows
+// over with them, by vertices a unit):
+//   k = 2, whose degree-proportional kernel is cheap, 500:  n = 36000 490 1.31, n = 65000 490 1.97, but n = 33000 656 0.93;
+//   k = 3, 1500:  n = 36000 1480 0.98, n = 65000 1480 1.32, but n = 65536 2250 0.74;
+//   k >= 4, 4000, from k = 17 on 3300:  3900 n = 36000, k = 4 4.6, k = 8 2.6, k = 12 1.33, k = 24 0.89 (2500 1.26).
+// us a move: G(65536, 0.02), k = 3 8.2 -> 4.0; G(40000, 0.05), k = 6 35.8 -> 3.4; G(65536, 0.01), k = 9 61.6 -> 23.3.
 bool PreferWindowWide(int n, int k, int64_t edges) {
   const double p = 2.0 * (double)edges / ((double)n * (n - 1));
   const double width = 2.8 * std::sqrt(std::max(0.0, n * p * (1.0 - p) / k));
-  return n <= (k == 2 ? 500.0 : k == 3 ? 1500.0 : 4000.0) * width;
+  return n <= (k == 2 ? 500.0 : k == 3 ? 1500.0 : k <= 16 ? 4000.0 : 3300.0) * width;
 }
 
 // Whether open twins by the thousand keep a graph from the windows: a move raises the gains of the moved vertex's twins, the

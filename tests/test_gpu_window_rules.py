@@ -125,3 +125,20 @@ def test_edge_count_beyond_32_bits(ccb, oracle, cuda_device, n, k):
     got = ccb.SolveGpu(ccb.Graph(n, bits, edges + (3 << 30)), ccb.PbilsParams(**p))
     assert (got.objective - (3 << 30), got.accepted_moves) == (want.objective, want.accepted_moves)
     assert np.array_equal(got.labels, want.labels)
+
+
+# Sparse graphs, whose gains are few: the other side of the width line against each descent that the windows replaced
+@pytest.mark.parametrize("n,k,density,windowed", [
+    (1400, 2, 0.2, True), (1400, 2, 0.05, False), (2048, 8, 0.05, True), (2048, 8, 0.01, False),
+    (2049, 2, 0.05, True), (2049, 2, 0.005, False), (4096, 8, 0.01, True), (4096, 8, 0.004, False),
+    (4097, 2, 0.004, True), (4200, 2, 0.0015, False), (4200, 3, 0.0022, True), (9000, 3, 0.0028, True), (9000, 3, 0.002, False),
+    (2000, 32, 0.0045, True), (2000, 32, 0.0022, False), (3001, 32, 0.0027, True)])
+def test_route_follows_the_width_of_the_gains(ccb, oracle, cuda_device, n, k, density, windowed):
+    bits, edges = oracle.erdos_renyi(n, density, n + k)
+    p = dict(k=k, population=2, iterations=1, early_stop=10, seed=4)
+    solver = ccb.Solver(ccb.DeviceGraph(ccb.Graph(n, bits, edges)), ccb.PbilsParams(**p))
+    assert solver.describe().startswith("windowed") == windowed, solver.describe()
+    got = solver.pbils(ccb.PbilsParams(**p))
+    want = oracle.pbils(bits, edges, make_params(**p))
+    assert (got.objective, got.accepted_moves) == (want.objective, want.accepted_moves)
+    assert np.array_equal(got.labels, want.labels)
