@@ -153,7 +153,8 @@ const char* ccb_solver_describe(const ccb_solver* solver);
 void ccb_solver_destroy(ccb_solver* solver);
 
 /* Per-kernel timing of the last solve (CUDA events around each launch; enabled by
- * ccb_solver_set_profiling).  Times in milliseconds, launches counted. */
+ * ccb_solver_set_profiling).  Times in milliseconds, launches counted.  Populations of at most 256 whose rebuild
+ * is by popcount record in the rebuild's launch, which counts as a rebuild (record: the initial one alone). */
 typedef struct ccb_kernel_stats {
   double descent_ms;
   double rebuild_ms;
