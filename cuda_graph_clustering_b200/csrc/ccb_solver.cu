@@ -316,9 +316,10 @@ size_t NextBytes(const Plan& plan, int n, int k, int ld, int pop) {
 }
 
 // `slots`: the slots whose descents share the device (the population, or what a batch or server runs together); windows =
-// false: never the windowed descent.
+// false: never the windowed descent; batched: for the batched engines, whose flow kernels need up to 1.5 KB of static shared
+// memory beside a streamed state (the plain kernels 0.5 KB).
 Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const Device& dev, int pop, int64_t edges,
-              const OpenTwins& twins, int slots, bool windows = true) {
+              const OpenTwins& twins, int slots, bool batched, bool windows = true) {
   Plan p;
   p.wide = n > CCB_MAX_VERTICES_NARROW || ls_kernel == CCB_LS_WIDE;
   p.threads = DescentThreads(n, p.wide);
@@ -350,7 +351,7 @@ Plan MakePlan(int n, int pitch, int k, int ld, int kpad, int ls_kernel, const De
       sk.smem_bytes = RegistersSmem(n, pitch, sk.smem_rows);
     } else {
       sk.threads = 1024;
-      sk.smem_state = SmallKSmem(k, n, pitch, ld, sk.threads, true, false) <= limit;
+      sk.smem_state = SmallKSmem(k, n, pitch, ld, sk.threads, true, false) + (batched ? 1024 : 0) <= limit;
       sk.smem_rows = false;
       sk.smem_bytes = SmallKSmem(k, n, pitch, ld, sk.threads, sk.smem_state, false);
       if (!sk.smem_state && kClusterDescent) {
@@ -764,7 +765,7 @@ ccb_solver* MakeSolver(const ccb_graph* g, int k, int pop, int ls_kernel, bool p
   size_t next_bytes = 0, bytes = 0;
   const auto plan = [&](bool windows) {
     s->plan = MakePlan(g->n, g->pitch, k, s->ld, s->kpad, ls_kernel, s->device, pop, g->edges, g->twins,
-                       plain ? pop : slots, windows);
+                       plain ? pop : slots, !plain, windows);
     // k = 2, 3 wide on a sparse graph (average degree <= n / 8): work per move follows the degree, not n
     s->plan.sparse = s->plan.packed_wide && 2.0 * (double)g->edges <= (double)g->n * g->n / 8.0;
     PlanSmem16(*s);
@@ -1783,10 +1784,10 @@ size_t RequestBytes(const ccb_server& sv, uint32_t n, const ccb_params& p) {
   const int kpad = (p.k + 3) / 4 * 4;
   // The descent, and with it its scratch, depends on the graph's density, not known before a generated graph's
   // admission, and on the load: the larger of both.
-  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0, OpenTwins(), 0,
+  const Plan plan = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population, 0, OpenTwins(), 0, true,
                              false);
   const Plan dense = MakePlan((int)n, pitch, p.k, ld, kpad, CCB_LS_AUTO, sv.device, p.population,
-                              (int64_t)n * (n - 1) / 4, OpenTwins(), 0);
+                              (int64_t)n * (n - 1) / 4, OpenTwins(), 0, true);
   const size_t labels = (size_t)p.population * ld;
   const size_t gb = plan.wide ? 4 : 2;
   const size_t next = std::max(NextBytes(plan, (int)n, p.k, ld, p.population),
@@ -1908,7 +1909,7 @@ bool BatchedKernelsTake(const ccb_server& sv, const ccb_server::Request& r) {
   const int pitch = std::max(4, (words + 3) / 4 * 4);
   const int ld = std::max(32, ((int)r.n + 31) / 32 * 32);
   const Plan pl = MakePlan((int)r.n, pitch, r.params.k, ld, (r.params.k + 3) / 4 * 4, CCB_LS_AUTO, sv.device,
-                           r.params.population, 0, OpenTwins(), 0);
+                           r.params.population, 0, OpenTwins(), 0, true);
   return !pl.wide && (pl.small_k || pl.incremental);
 }
 
@@ -2476,7 +2477,7 @@ ccb_solver& CachedSolver(const uint32_t* bits, uint32_t n, uint32_t words_per_ro
     // the windowed descent depends on the density and the ties: a change needs other buffers
     const ccb_solver& old = *c.solver;
     const bool windows = MakePlan(old.n, g.pitch, k, old.ld, old.kpad, ls_kernel, old.device, pop, g.edges, g.twins,
-                                  pop).sk.window;
+                                  pop, false).sk.window;
     if (windows != old.plan.sk.window && !(windows && old.windows_refused)) {
       c.solver.reset();
       c.solver.reset(MakeSolver(&g, k, pop, ls_kernel));

@@ -114,3 +114,20 @@ def test_tuned_batch_of_sparse_graphs_takes_the_global_form(ccb, cuda_device, th
             _same(batch.result(i), ccb.Solver(graph, p).pbils(p))
     finally:
         ccb.set_tuning(before)
+
+
+@pytest.mark.parametrize("engine", ["lockstep", "flow"])
+@pytest.mark.parametrize("n,k", [(14450, 8), (28910, 3)])
+def test_batched_stream_at_the_edge_of_shared_memory(ccb, cuda_device, engine, n, k):
+    """A streamed state of 226 KB fits beside the plain kernel's static shared memory, not beside the flow kernel's: the
+    batch streams it from L2."""
+    graph = ccb.DeviceGraph.erdos_renyi(n, 0.0004, 7)
+    p = ccb.PbilsParams(k=k, population=3, iterations=1, early_stop=5, seed=2)
+    plain = ccb.Solver(graph, p)
+    assert plain.describe().startswith("packed k <= 8, streamed from shared memory")
+    batch = ccb.Batch(engine=engine)
+    i = batch.add(graph, p)
+    batch.run()
+    assert "stream k=%d threads=1024 vpt=4 smem=0" % k in batch.describe(), batch.describe()
+    _same(batch.result(i), plain.pbils(p))
+    batch.close()
